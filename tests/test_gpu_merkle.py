@@ -116,6 +116,19 @@ def test_vs_oracle(zk, oracle, ht, nl, ls, ch):
     assert np.array_equal(c, c2) and np.array_equal(d, d2)
 
 
+@pytest.mark.parametrize("ht", [0, 3, 4])
+@pytest.mark.parametrize("nl,ls,ch", [(64, 17, 0), (1 << 14, 9, 2), (1 << 15, 12, 3)])
+def test_edge_words_vs_oracle(zk, oracle, ht, nl, ls, ch):
+    """Leaves of the words at the edges of the reductions and of the layers' 32-bit halves, on each thread layout."""
+    edge = np.array([0, 1, 0xFFFFFFFE, 0xFFFFFFFF, 1 << 32, 1 << 63, 0xFFFFFFFEFFFFFFFF, 0xFFFFFFFF00000000],
+                    dtype=np.uint64)  # all below p
+    i = np.arange(nl * ls, dtype=np.uint64)
+    leaves = edge[((i * np.uint64(7) + i // np.uint64(5) + i // np.uint64(31)) % np.uint64(len(edge))).astype(np.int64)]
+    d, c = gpu_tree(zk, leaves, ls, ch, ht)
+    d2, c2 = oracle.merkle_fill(leaves, ls, ch, ht)
+    assert np.array_equal(c, c2) and np.array_equal(d, d2)
+
+
 def test_cpu_entry_point(zk, oracle):
     """fill_digests_buf_linear_cpu: host buffers, same tree."""
     nl, ls, ch = 1024, 135, 4

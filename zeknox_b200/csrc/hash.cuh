@@ -25,56 +25,212 @@
 namespace zk {
 
 // ---------------------------------------------------- exact FP64 layers
-// The linear layers of both Poseidon variants have small non-negative integer
-// coefficients.  They run on the FP64 pipe (full rate on sm_100), next to the
-// integer pipes that carry the S-box products: each lane is split into its two
-// 32-bit halves, each half-vector goes through the layer in doubles, and every
-// product and partial sum is an integer (or half-integer) far below 2^53, so
+// The linear layers with small integer coefficients run on the FP64 pipe, next
+// to the integer pipes that carry the S-box products: each lane is split into
+// its two 32-bit halves, each half-vector goes through the layer in doubles,
+// and every product and partial sum is an integer below 2^53 in magnitude, so
 // the FP64 arithmetic is exact.
 //
-// No int<->double conversion instruction is used.  A 32-bit x enters as the
-// double whose bit pattern is 0x43300000:x, which is 2^52 + x; a result v
-// (0 <= v < 2^41) leaves as the double 2^52 + v, whose bit pattern is
-// kMagicBits + v.  Those two offsets are cancelled by subtracting
-// kMagicAdj = kMagicBits * (1 + 2^32) mod p from the constant that is added
-// in the same reduction (the next round's constants), so the constant tables
-// used there are stored pre-adjusted.
-constexpr double kMagic = 4503599627370496.0;  // 2^52
-constexpr uint64_t kMagicBits = 0x4330000000000000ull;
+// No conversion instruction is used: the 64-bit pattern of a non-negative
+// integer n < 2^53 read as a double is n 2^-1074 (a denormal, and from 2^52 on
+// the first normals), so integers go in as the word pair (x, 0) and results
+// come out as their own bit pattern.  FP64 runs at the same rate on denormals
+// (63.5 DFMA per clock and SM measured either way).
+//
+// Cost model behind the splits below (measured on the Poseidon leaf kernel): a
+// scheduler slot per instruction, two for an FP64 instruction and two for a
+// 32 x 32 -> 64-bit multiply; the kernels run at 90 % or more of that.
 __host__ __device__ constexpr uint64_t cx_canon(uint64_t a) { return a >= ZK_P ? a - ZK_P : a; }
-constexpr uint64_t cx_add_mod(uint64_t a, uint64_t b) {  // a, b < p
+__host__ __device__ constexpr uint64_t cx_add_mod(uint64_t a, uint64_t b) {  // a, b < p
     return a >= ZK_P - b ? a - (ZK_P - b) : a + b;
 }
-constexpr uint64_t cx_sub_mod(uint64_t a, uint64_t b) { return a >= b ? a - b : a + (ZK_P - b); }
-// kMagicBits * 2^32 = hi32 * 2^64 = hi32 * (2^32 - 1) (mod p) because its low word is zero.
-constexpr uint64_t kMagicAdj = cx_add_mod(kMagicBits, (kMagicBits >> 32 << 32) - (kMagicBits >> 32));
-static_assert((kMagicBits & 0xffffffffull) == 0 && kMagicAdj == 0x865fffffbcd00000ull, "magic constants");
-constexpr uint64_t kMagicNeg = cx_sub_mod(0, kMagicAdj);  // added where no constant follows
+__host__ __device__ constexpr uint64_t cx_sub_mod(uint64_t a, uint64_t b) { return a >= b ? a - b : a + (ZK_P - b); }
+constexpr uint64_t cx_mul_mod(uint64_t a, uint64_t b) {  // a < p, any b
+    uint64_t r = 0;
+    for (int i = 63; i >= 0; i--) {
+        r = cx_add_mod(r, r);
+        if (b >> i & 1) r = cx_add_mod(r, a);
+    }
+    return r;
+}
+constexpr uint64_t cx_mont(uint64_t a) { return cx_mul_mod(0xffffffffull, cx_canon(a)); }  // a 2^64 mod p
 
 struct RcTable {
     uint64_t v[360];
 };
-constexpr RcTable magic_adjusted(RcTable t) {
-    for (int i = 0; i < 360; i++) t.v[i] = cx_sub_mod(cx_canon(t.v[i]), kMagicAdj);
-    return t;
+
+// Circulant layers C[r][k] = c[(k - r) mod 12] plus diag(d, 0, ..., 0).  In 6x6
+// blocks C = [[A, B], [B, A]], so with u = x_lo + x_hi and w = x_lo - x_hi
+// (x_lo = lanes 0-5, x_hi = lanes 6-11),
+//   2 (C x)_lo = (A + B) u + (A - B) w,   2 (C x)_hi = (A + B) u - (A - B) w,
+// which takes 72 multiply-adds per half-vector instead of 144.  The products of
+// such matrices split the same way, with (A + B)^2 and (A - B)^2.  u and w are
+// formed by integer adds that leave a ready word pair; w carries an offset of
+// 2^32 to stay non-negative, which the constants added to the results take
+// out again (circ_offset).
+template <class H>
+struct Circ {  // H::c(j), j in 0..11: the first row; H::d0(): the diagonal term
+    __host__ __device__ static constexpr int at(int j) { return H::c(((j % 12) + 12) % 12); }
+    __host__ __device__ static constexpr int at2(int j) {  // first row of C^2
+        int v = 0;
+        for (int i = 0; i < 12; i++) v += at(i) * at(j - i);
+        return v;
+    }
+    // entries of A + B and A - B, of C (N = 1) or C^2 (N = 2)
+    template <int N>
+    __host__ __device__ static constexpr int p(int r, int k) {
+        return N == 1 ? at(k - r) + at(k + 6 - r) : at2(k - r) + at2(k + 6 - r);
+    }
+    template <int N>
+    __host__ __device__ static constexpr int q(int r, int k) {
+        return N == 1 ? at(k - r) - at(k + 6 - r) : at2(k - r) - at2(k + 6 - r);
+    }
+    // what the offset of w adds to output row r of either half-vector
+    template <int N>
+    static constexpr int64_t offset(int r) {
+        int64_t v = 0;
+        for (int k = 0; k < 6; k++) v += q<N>(r % 6, k);
+        return (r < 6 ? v : -v) * (1ll << 31);
+    }
+};
+
+// The starting values (lo, hi) of an output's two accumulators, as integers:
+// lo + hi 2^32 = k (mod p), less the w offset; `bias` keeps both accumulators
+// positive throughout.
+struct KPair {
+    uint64_t lo, hi;
+};
+constexpr KPair make_kpair(uint64_t k, int64_t offset, uint64_t bias) {
+    const uint64_t b2 = cx_add_mod(cx_canon(bias), cx_mul_mod(cx_canon(bias), 1ull << 32));
+    const uint64_t d = cx_sub_mod(cx_canon(k), b2);
+    return KPair{bias - (uint64_t)offset + (d & 0xffffffffull), bias - (uint64_t)offset + (d >> 32)};
 }
 
-// Poseidon: the next round's constant c goes into the FP64 accumulators
-// instead of the integer reduction.  With m = (c - kMagicAdj) mod p, the low
-// and high half-vector outputs of round rnd start from 2^52 + (m mod 2^32) and
-// 2^52 + floor(m / 2^32) (exact: both below 2^53), so that
-// bits(lo) + bits(hi) * 2^32 = MDS x + c (mod p).  Round 29 has no constant.
-struct MdsK {
-    double v[30][2][12];
-};
-constexpr MdsK make_mds_k(RcTable rc) {
-    MdsK t{};
-    for (int rnd = 0; rnd < 30; rnd++)
-        for (int r = 0; r < 12; r++) {
-            const uint64_t m = cx_sub_mod(rnd < 29 ? cx_canon(rc.v[12 * (rnd + 1) + r]) : 0, kMagicAdj);
-            t.v[rnd][0][r] = kMagic + (double)(m & 0xffffffffull);
-            t.v[rnd][1][r] = kMagic + (double)(m >> 32);
+__device__ __forceinline__ double int_dbl(uint64_t n) { return __longlong_as_double((long long)n); }
+__device__ __forceinline__ double word_dbl(uint32_t x) { return __hiloint2double(0, (int)x); }
+__device__ __forceinline__ uint64_t dbl_int(double v) { return (uint64_t)__double_as_longlong(v); }
+// a + b and a - b + 2^32 as doubles
+__device__ __forceinline__ double sum_dbl(uint32_t a, uint32_t b) {
+    uint32_t lo, hi;
+    asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, 0, 0;" : "=r"(lo), "=r"(hi) : "r"(a), "r"(b));
+    return __hiloint2double((int)hi, (int)lo);
+}
+__device__ __forceinline__ double diff_dbl(uint32_t a, uint32_t b) {
+    uint32_t lo, hi;
+    asm("sub.cc.u32 %0, %2, %3;\n\tsubc.u32 %1, 1, 0;" : "=r"(lo), "=r"(hi) : "r"(a), "r"(b));
+    return __hiloint2double((int)hi, (int)lo);
+}
+__device__ __forceinline__ uint32_t half_of(uint64_t x, int h) { return h ? (uint32_t)(x >> 32) : (uint32_t)x; }
+
+// Half h of the lanes s through the layer: o[r] = k[r] + (C x)[r] + [r = 0] d x[0].
+template <class H>
+__device__ __forceinline__ void circ_half(const uint64_t s[12], int h, double o[12], const uint64_t *k) {
+    using C = Circ<H>;
+    double u[6], w[6];
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        u[i] = sum_dbl(half_of(s[i], h), half_of(s[i + 6], h));
+        w[i] = diff_dbl(half_of(s[i], h), half_of(s[i + 6], h));
+    }
+#pragma unroll
+    for (int r = 0; r < 6; r++) {
+        double pa = (double)C::template p<1>(r, 0) * u[0], qa = (double)C::template q<1>(r, 0) * w[0];
+#pragma unroll
+        for (int c = 1; c < 6; c++) {
+            pa = fma((double)C::template p<1>(r, c), u[c], pa);
+            qa = fma((double)C::template q<1>(r, c), w[c], qa);
         }
+        o[r] = fma(0.5, pa + qa, int_dbl(k[r]));
+        if (H::d0() != 0 && r == 0) o[0] = fma((double)H::d0(), word_dbl(half_of(s[0], h)), o[0]);
+        o[r + 6] = fma(0.5, pa - qa, int_dbl(k[r + 6]));
+    }
+}
+template <class H>
+__device__ __forceinline__ void circ_layer(uint64_t s[12], const uint64_t (*k)[12]) {
+    double lo[12], hi[12];
+    circ_half<H>(s, 0, lo, k[0]);
+    circ_half<H>(s, 1, hi, k[1]);
+#pragma unroll
+    for (int r = 0; r < 12; r++) s[r] = pr_reduce_split(dbl_int(lo[r]), dbl_int(hi[r]));
+}
+
+// ------------------------------------------------------------ Poseidon
+// MDS = C + diag(8, 0, ..., 0), C circulant.
+struct PoseidonMds {
+    __host__ __device__ static constexpr int c(int j) {
+        constexpr uint32_t circ[12] = {ZK_POSEIDON_MDS_CIRC_LIST};
+        return (int)circ[j];
+    }
+    __host__ __device__ static constexpr int d0() {
+        constexpr uint32_t diag[12] = {ZK_POSEIDON_MDS_DIAG_LIST};
+        return (int)diag[0];
+    }
+};
+using PoseidonCirc = Circ<PoseidonMds>;
+constexpr bool diag_only_lane0() {
+    constexpr uint32_t diag[12] = {ZK_POSEIDON_MDS_DIAG_LIST};
+    for (int i = 1; i < 12; i++)
+        if (diag[i]) return false;
+    return true;
+}
+static_assert(diag_only_lane0(), "the MDS layer below assumes diag(d, 0, ..., 0)");
+
+// Round r adds its 12 constants, applies x^7 (all lanes in rounds 0-3 and
+// 26-29, lane 0 otherwise) and the MDS layer M = C + d e0 e0^T.  Constants of
+// round r + 1 are added inside round r's layer.
+//
+// The 22 partial rounds run two at a time.  With x the state, x0' = S(x0),
+// c, c' the next two rounds' constants, y0 = (M x')_0 + c_0 and y0' = S(y0):
+//   M (M x' + c + (y0' - y0) e0) + c'
+//     = C^2 x' + g C e0 + d y0' e0 + (C c + c'),    g = d x0' + y0' - y0,
+// one layer's work for two rounds plus one row for y0 and one column for g.
+// C^2 has entries below 2^13 and row sums of 2^16, so every sum stays below
+// 2^50.  g and y0 stay split in (unreduced) halves.
+struct PoseidonTab {
+    uint64_t full[8][2][12];   // layers of rounds 0-3 and 26-29 (no constants after 29)
+    uint64_t pair[11][2][12];  // layers of round pairs (4, 5) .. (24, 25)
+    uint64_t mid[11][2];       // y0 of each pair
+    uint64_t rc0[12];          // round 0, added before the first S-box
+    // the six-thread form's rows t of A + B and A - B (for C and C^2), and C e0 at rows t and t + 6
+    double rows[6][26];
+};
+constexpr uint64_t kFullBias = 1ull << 40;  // above the w offset of C: 113 * 2^31
+constexpr uint64_t kPairBias = 1ull << 48;  // above 41 * 2^42 of -g and the w offset of C^2
+constexpr PoseidonTab make_poseidon_tab(RcTable rc) {
+    PoseidonTab t{};
+    for (int i = 0; i < 12; i++) t.rc0[i] = cx_canon(rc.v[i]);
+    for (int f = 0; f < 8; f++) {
+        const int rnd = f < 4 ? f : 22 + f;
+        for (int r = 0; r < 12; r++) {
+            const KPair k = make_kpair(rnd < 29 ? rc.v[12 * (rnd + 1) + r] : 0, PoseidonCirc::offset<1>(r), kFullBias);
+            t.full[f][0][r] = k.lo;
+            t.full[f][1][r] = k.hi;
+        }
+    }
+    for (int q = 0; q < 11; q++) {
+        const uint64_t *c = &rc.v[12 * (5 + 2 * q)], *c2 = &rc.v[12 * (6 + 2 * q)];
+        const KPair m = make_kpair(c[0], PoseidonCirc::offset<1>(0), kFullBias);
+        t.mid[q][0] = m.lo;
+        t.mid[q][1] = m.hi;
+        for (int r = 0; r < 12; r++) {
+            uint64_t v = cx_canon(c2[r]);
+            for (int j = 0; j < 12; j++)
+                v = cx_add_mod(v, cx_mul_mod(cx_canon(c[j]), (uint64_t)PoseidonCirc::at(j - r)));
+            const KPair k = make_kpair(v, PoseidonCirc::offset<2>(r), kPairBias);
+            t.pair[q][0][r] = k.lo;
+            t.pair[q][1][r] = k.hi;
+        }
+    }
+    for (int r = 0; r < 6; r++) {
+        for (int k = 0; k < 6; k++) {
+            t.rows[r][k] = PoseidonCirc::p<1>(r, k);
+            t.rows[r][6 + k] = PoseidonCirc::q<1>(r, k);
+            t.rows[r][12 + k] = PoseidonCirc::p<2>(r, k);
+            t.rows[r][18 + k] = PoseidonCirc::q<2>(r, k);
+        }
+        t.rows[r][24] = PoseidonCirc::at(-r);
+        t.rows[r][25] = PoseidonCirc::at(-r - 6);
+    }
     return t;
 }
 
@@ -83,28 +239,16 @@ constexpr MdsK make_mds_k(RcTable rc) {
 // block's shared-memory copy of the __device__ twin (latency-bound kernels
 // with a few warps, which would otherwise wait on a constant-cache miss in
 // every round).
-struct PoseidonTab {
-    MdsK mdsk;         // next-round constants inside the MDS accumulators
-    uint64_t rc0[12];  // round 0, added before the first S-box
-};
 struct Poseidon2Tab {
-    RcTable rcm;        // external rounds: adjusted for the magic offsets
-    RcTable rc;         // internal rounds (lane 0) and the first external round after them
-    uint64_t diag[12];  // internal-layer diagonal
+    uint64_t rc[31][12];  // constants added after each layer: [r] before round r's S-box, [30] zero
+    uint64_t diag[12];    // internal-layer diagonal, times 2^64
 };
 struct KeccakTab {};
-constexpr PoseidonTab make_poseidon_tab(RcTable rc) {
-    PoseidonTab t{};
-    t.mdsk = make_mds_k(rc);
-    for (int i = 0; i < 12; i++) t.rc0[i] = cx_canon(rc.v[i]);
-    return t;
-}
 constexpr Poseidon2Tab make_poseidon2_tab(RcTable rc) {
     Poseidon2Tab t{};
-    t.rcm = magic_adjusted(rc);
-    t.rc = rc;
+    for (int i = 0; i < 360; i++) t.rc[i / 12][i % 12] = cx_canon(rc.v[i]);
     constexpr uint64_t d[12] = {ZK_POSEIDON2_DIAG_LIST};
-    for (int i = 0; i < 12; i++) t.diag[i] = d[i];
+    for (int i = 0; i < 12; i++) t.diag[i] = cx_mont(d[i]);
     return t;
 }
 __constant__ PoseidonTab c_poseidon = make_poseidon_tab(RcTable{{ZK_POSEIDON_RC_LIST}});
@@ -114,104 +258,49 @@ __device__ Poseidon2Tab g_poseidon2 = make_poseidon2_tab(RcTable{{ZK_POSEIDON2_R
 __constant__ uint64_t c_keccak_rc[24] = {ZK_KECCAK_RC_LIST};
 __constant__ KeccakTab c_keccak_tab;
 
-__device__ __forceinline__ double magic_in(uint32_t x) { return __hiloint2double(0x43300000, (int)x); }
-__device__ __forceinline__ uint64_t magic_out(double v) { return (uint64_t)__double_as_longlong(v); }
-
-// s[r] <- (lo[r] + hi[r] * 2^32 + c[r]) mod p (partially reduced), where lo, hi
-// are the magic-offset outputs of a layer and cm the adjusted constants
-// (nullptr: no constant).
-__device__ __forceinline__ void magic_combine(uint64_t s[12], const double lo[12], const double hi[12],
-                                              const uint64_t *cm) {
+// Two partial rounds (the pair q), see above.
+__device__ __forceinline__ void poseidon_pair(uint64_t s[12], int q, const PoseidonTab &tab) {
+    using C = PoseidonCirc;
+    constexpr double d0 = (double)PoseidonMds::d0();
+    double u[2][6], w[2][6], y0[2], lo[12];
+    s[0] = pr_pow7(s[0]);
 #pragma unroll
-    for (int r = 0; r < 12; r++) s[r] = pr_reduce_split(magic_out(lo[r]), magic_out(hi[r]), cm ? cm[r] : kMagicNeg);
-}
-
-// ------------------------------------------------------------ Poseidon
-// MDS = C + diag(8, 0, ..., 0), C circulant with C[r][k] = circ[(k - r) mod 12].
-// In 6x6 blocks C = [[A, B], [B, A]], so with u = x_lo + x_hi, w = x_lo - x_hi
-// (x_lo = lanes 0-5, x_hi = lanes 6-11):
-//   2 (C x)_lo = (A + B) u + (A - B) w,   2 (C x)_hi = (A + B) u - (A - B) w,
-// which takes 72 multiply-adds per half-vector instead of 144.
-#define ZK_MDS_TABLES                                                  \
-    constexpr uint32_t circ[12] = {ZK_POSEIDON_MDS_CIRC_LIST};         \
-    constexpr uint32_t diag[12] = {ZK_POSEIDON_MDS_DIAG_LIST};
-constexpr bool diag_only_lane0() {
-    ZK_MDS_TABLES
-    for (int i = 1; i < 12; i++)
-        if (diag[i]) return false;
-    return circ[0] > 0;
-}
-static_assert(diag_only_lane0(), "the MDS layer below assumes diag(d, 0, ..., 0)");
-__host__ __device__ constexpr int mds_diag0() {
-    ZK_MDS_TABLES
-    return (int)diag[0] + 0 * (int)circ[0];
-}
-__host__ __device__ constexpr int mds_p2(int r, int k) {  // A + B, plus d on (0, 0)
-    ZK_MDS_TABLES
-    return (int)(circ[(k - r + 12) % 12] + circ[(k + 6 - r + 12) % 12]) + (r == 0 && k == 0 ? (int)diag[0] : 0);
-}
-__host__ __device__ constexpr int mds_q2(int r, int k) {  // A - B, plus d on (0, 0)
-    ZK_MDS_TABLES
-    return (int)circ[(k - r + 12) % 12] - (int)circ[(k + 6 - r + 12) % 12] + (r == 0 && k == 0 ? (int)diag[0] : 0);
-}
-#undef ZK_MDS_TABLES
-
-// Coefficients of the circulant split for one hasher's MDS.
-struct PoseidonCirc {
-    __host__ __device__ static constexpr int p2(int r, int k) { return mds_p2(r, k); }
-    __host__ __device__ static constexpr int q2(int r, int k) { return mds_q2(r, k); }
-    __host__ __device__ static constexpr int d0() { return mds_diag0(); }
-};
-
-// One half-vector: a[i] = 2^52 + x[i] in, o[r] = k[r] + (M x)[r] out, M the
-// circulant (plus diag(d0, 0, ...)) of C.
-template <class C>
-__device__ __forceinline__ void circ12_half(const double a[12], double o[12], const double *k) {
-    double u[6], w[6], x6 = 0.0;
+    for (int h = 0; h < 2; h++) {
+        double pa = 0, qa = 0;
 #pragma unroll
-    for (int i = 0; i < 6; i++) {
-        const double t = a[i + 6] - kMagic;  // x_hi[i]
-        if (i == 0) x6 = t;
-        w[i] = a[i] - a[i + 6];              // exact: both in [2^52, 2^53)
-        u[i] = fma(2.0, t, w[i]);
-    }
-#pragma unroll
-    for (int r = 0; r < 6; r++) {
-        // Lanes 0 and 6 (u[0], w[0]) last: in a partial round only lane 0 has
-        // just left the S-box, so the other terms need not wait for it.
-        double pa = (double)C::p2(r, 1) * u[1], qa = (double)C::q2(r, 1) * w[1];
-#pragma unroll
-        for (int c = 2; c < 6; c++) {
-            pa = fma((double)C::p2(r, c), u[c], pa);
-            qa = fma((double)C::q2(r, c), w[c], qa);
+        for (int i = 5; i >= 0; i--) {  // lane 0, which has just left the S-box, last
+            u[h][i] = sum_dbl(half_of(s[i], h), half_of(s[i + 6], h));
+            w[h][i] = diff_dbl(half_of(s[i], h), half_of(s[i + 6], h));
+            pa = fma((double)C::p<1>(0, i), u[h][i], pa);
+            qa = fma((double)C::q<1>(0, i), w[h][i], qa);
         }
-        pa = fma((double)C::p2(r, 0), u[0], pa);
-        qa = fma((double)C::q2(r, 0), w[0], qa);
-        // The (0, 0) terms carry d (u + w) = 2 d x_lo[0] into lane 0; lane 6
-        // must not get d (u - w) = 2 d x_hi[0], so it is taken out again.
-        double d = pa - qa;
-        if constexpr (C::d0() != 0) {
-            if (r == 0) d = fma(-2.0 * (double)C::d0(), x6, d);
-        }
-        o[r] = fma(0.5, pa + qa, k[r]);
-        o[r + 6] = fma(0.5, d, k[r + 6]);
+        y0[h] = fma(0.5, pa + qa, fma(d0, word_dbl(half_of(s[0], h)), int_dbl(tab.mid[q][h])));
     }
-}
-__device__ __forceinline__ void poseidon_mds_half(const double a[12], double o[12], const double *k) {
-    circ12_half<PoseidonCirc>(a, o, k);
-}
-
-// s <- MDS s + c, c being round rnd + 1's constants (none after round 29).
-__device__ __forceinline__ void poseidon_mds(uint64_t s[12], int rnd, const PoseidonTab &tab) {
-    double a[12], lo[12], hi[12];
+    const uint64_t x0 = s[0], y = pr_pow7(pr_reduce_split(dbl_int(y0[0]), dbl_int(y0[1])));
 #pragma unroll
-    for (int i = 0; i < 12; i++) a[i] = magic_in((uint32_t)s[i]);
-    poseidon_mds_half(a, lo, tab.mdsk.v[rnd][0]);
+    for (int h = 0; h < 2; h++) {
+        const double yp = word_dbl(half_of(y, h));
+        const double g = fma(d0, word_dbl(half_of(x0, h)), yp - y0[h]);
 #pragma unroll
-    for (int i = 0; i < 12; i++) a[i] = magic_in((uint32_t)(s[i] >> 32));
-    poseidon_mds_half(a, hi, tab.mdsk.v[rnd][1]);
+        for (int r = 0; r < 6; r++) {
+            double pa = (double)C::p<2>(r, 5) * u[h][5], qa = (double)C::q<2>(r, 5) * w[h][5];
 #pragma unroll
-    for (int r = 0; r < 12; r++) s[r] = pr_reduce_split_nc(magic_out(lo[r]), magic_out(hi[r]));
+            for (int c = 4; c >= 0; c--) {
+                pa = fma((double)C::p<2>(r, c), u[h][c], pa);
+                qa = fma((double)C::q<2>(r, c), w[h][c], qa);
+            }
+            double o0 = fma((double)C::at(-r), g, fma(0.5, pa + qa, int_dbl(tab.pair[q][h][r])));
+            const double o6 = fma((double)C::at(-r - 6), g, fma(0.5, pa - qa, int_dbl(tab.pair[q][h][r + 6])));
+            if (r == 0) o0 = fma(d0, yp, o0);
+            if (h == 0) {
+                lo[r] = o0;
+                lo[r + 6] = o6;
+            } else {
+                s[r] = pr_reduce_split(dbl_int(lo[r]), dbl_int(o0));
+                s[r + 6] = pr_reduce_split(dbl_int(lo[r + 6]), dbl_int(o6));
+            }
+        }
+    }
 }
 
 // x^7 on all 12 lanes.  W = 4: three passes over 4 lanes with a rotation
@@ -240,18 +329,20 @@ __device__ __forceinline__ void pow7_all(uint64_t s[12]) {
 }
 
 // The permutation on a partially reduced state (outputs partially reduced).
-// Round r adds its 12 constants, applies x^7 (all lanes in rounds 0-3 and
-// 26-29, lane 0 otherwise) and the MDS layer; each round's constants are
-// added inside the previous round's MDS reduction.
 template <int W = 4>
 __device__ __forceinline__ void poseidon_permute(uint64_t s[12], const PoseidonTab &tab = c_poseidon) {
 #pragma unroll
     for (int i = 0; i < 12; i++) s[i] = pr_add_c(s[i], tab.rc0[i]);
 #pragma unroll 1
-    for (int rnd = 0; rnd < 30; rnd++) {
-        if (rnd < 4 || rnd >= 26) pow7_all<W>(s);
-        else s[0] = pr_pow7(s[0]);
-        poseidon_mds(s, rnd, tab);
+    for (int half = 0; half < 2; half++) {
+#pragma unroll 1
+        for (int f = 0; f < 4; f++) {
+            pow7_all<W>(s);
+            circ_layer<PoseidonMds>(s, tab.full[4 * half + f]);
+        }
+        if (half) break;
+#pragma unroll 1
+        for (int q = 0; q < 11; q++) poseidon_pair(s, q, tab);
     }
 }
 
@@ -262,14 +353,14 @@ __device__ __forceinline__ void poseidon_permute(uint64_t s[12], const PoseidonT
 // M4 x is the 8-addition network of the Poseidon2 paper (Grassi, Khovratovich,
 // Schofnegger 2023, section 5.1): t0 = x0 + x1, t1 = x2 + x3, t2 = 2 x1 + t1,
 // t3 = 2 x3 + t0, t4 = 4 t1 + t3, t5 = 4 t0 + t2, M4 x = (t3 + t5, t5, t2 + t4, t4).
-__device__ __forceinline__ void poseidon2_external_half(const double a[12], double o[12]) {
+__device__ __forceinline__ void poseidon2_external_half(const uint64_t s[12], int h, double o[12]) {
     double y[12];
 #pragma unroll
     for (int b = 0; b < 3; b++) {
-        const double x0 = a[4 * b] - kMagic, x1 = a[4 * b + 1] - kMagic;
-        const double x2 = a[4 * b + 2] - kMagic, x3 = a[4 * b + 3] - kMagic;
-        const double t0 = x0 + x1, t1 = x2 + x3;
-        const double t2 = fma(2.0, x1, t1), t3 = fma(2.0, x3, t0);
+        const uint32_t x0 = half_of(s[4 * b], h), x1 = half_of(s[4 * b + 1], h);
+        const uint32_t x2 = half_of(s[4 * b + 2], h), x3 = half_of(s[4 * b + 3], h);
+        const double t0 = sum_dbl(x0, x1), t1 = sum_dbl(x2, x3);
+        const double t2 = fma(2.0, word_dbl(x1), t1), t3 = fma(2.0, word_dbl(x3), t0);
         const double t4 = fma(4.0, t1, t3), t5 = fma(4.0, t0, t2);
         y[4 * b] = t3 + t5;
         y[4 * b + 1] = t5;
@@ -278,65 +369,83 @@ __device__ __forceinline__ void poseidon2_external_half(const double a[12], doub
     }
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        const double sm = (y[j] + y[4 + j]) + (y[8 + j] + kMagic);
+        const double sm = (y[j] + y[4 + j]) + y[8 + j];
 #pragma unroll
         for (int b = 0; b < 3; b++) o[4 * b + j] = y[4 * b + j] + sm;
     }
 }
-
-__device__ __forceinline__ void poseidon2_external(uint64_t s[12], const uint64_t *cm) {
-    double a[12], lo[12], hi[12];
+__device__ __forceinline__ void poseidon2_external(uint64_t s[12], const uint64_t *c) {
+    double lo[12], hi[12];
+    poseidon2_external_half(s, 0, lo);
+    poseidon2_external_half(s, 1, hi);
 #pragma unroll
-    for (int i = 0; i < 12; i++) a[i] = magic_in((uint32_t)s[i]);
-    poseidon2_external_half(a, lo);
-#pragma unroll
-    for (int i = 0; i < 12; i++) a[i] = magic_in((uint32_t)(s[i] >> 32));
-    poseidon2_external_half(a, hi);
-    magic_combine(s, lo, hi, cm);
+    for (int r = 0; r < 12; r++) s[r] = pr_reduce_split_add(dbl_int(lo[r]), dbl_int(hi[r]), c[r]);
 }
 
-// x_i <- x_i * D_i + sum_j x_j (+ next round's constants): poseidon2.cu:131-146.
-// The sum of the 12 lanes is kept exact in 96 bits (carry chain).
-__device__ __forceinline__ void poseidon2_internal(uint64_t s[12], const uint64_t *c, const uint64_t *diag) {
-    uint32_t s0 = (uint32_t)s[0], s1 = (uint32_t)(s[0] >> 32), s2 = 0;
+// Internal layer, x_i <- x_i D_i + sum_j x_j (poseidon2.cu:131-146), and the
+// next round's constant (lane 0 only).  With R = 2^64, each lane is one
+// Montgomery reduction of x_i (D_i R) + (sum R mod p): the sum's two words
+// start the product's accumulators (mul_add_words), so adding it costs nothing
+// per lane.  R = 2^32 - 1 and 2^128 = -2^32, so (z2 z1 z0) R = (z0 - z2) 2^32 - z0 - z1.
+__device__ __forceinline__ uint64_t poseidon2_sum_mont(uint32_t z0, uint32_t z1, uint32_t z2) {
+    // z0 2^32 + (2^64 - 2^32 + 1) [= p] - z0 - z1 - z2 2^32, positive and below 2^65
+    uint32_t r0, r1;
+    asm("{\n\t"
+        ".reg .u32 a0, a1, b0, b1, k;\n\t"
+        "add.cc.u32 b0, %2, %3;\n\t"       // z0 + z1 + z2 2^32
+        "addc.u32 b1, %4, 0;\n\t"
+        "sub.cc.u32 a0, 0, b0;\n\t"        // z0 2^32 - that; a borrow adds p back
+        "subc.cc.u32 a1, %2, b1;\n\t"
+        "subc.u32 k, 0, 0;\n\t"
+        "sub.cc.u32 %0, a0, k;\n\t"
+        "subc.u32 %1, a1, 0;\n\t"
+        "}"
+        : "=r"(r0), "=r"(r1)
+        : "r"(z0), "r"(z1), "r"(z2));
+    return ((uint64_t)r1 << 32) | r0;
+}
+__device__ __forceinline__ uint64_t poseidon2_lane(uint64_t x, uint64_t d, uint64_t sum) {
+    uint32_t w[4];
+    mul_add_words(x, d, (uint32_t)sum, (uint32_t)(sum >> 32), w);
+    return mont_reduce(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ void poseidon2_internal(uint64_t s[12], uint64_t c0, const uint64_t *diag) {
+    uint32_t z0 = (uint32_t)s[0], z1 = (uint32_t)(s[0] >> 32), z2 = 0;  // the sum of the lanes, exact in 96 bits
 #pragma unroll
     for (int i = 1; i < 12; i++) {
         asm("add.cc.u32 %0, %0, %3;\n\t"
             "addc.cc.u32 %1, %1, %4;\n\t"
             "addc.u32 %2, %2, 0;"
-            : "+r"(s0), "+r"(s1), "+r"(s2)
+            : "+r"(z0), "+r"(z1), "+r"(z2)
             : "r"((uint32_t)s[i]), "r"((uint32_t)(s[i] >> 32)));
     }
+    const uint64_t sum = poseidon2_sum_mont(z0, z1, z2);
 #pragma unroll
-    for (int i = 0; i < 12; i++) {
-        uint32_t c0, c1, c2;
-        asm("add.cc.u32 %0, %3, %6;\n\t"
-            "addc.cc.u32 %1, %4, %7;\n\t"
-            "addc.u32 %2, %5, 0;"
-            : "=r"(c0), "=r"(c1), "=r"(c2)
-            : "r"(s0), "r"(s1), "r"(s2), "r"((uint32_t)c[i]), "r"((uint32_t)(c[i] >> 32)));
-        s[i] = pr_mul_add(s[i], diag[i], ((uint64_t)c1 << 32) | c0, c2);
-    }
+    for (int i = 0; i < 12; i++) s[i] = poseidon2_lane(s[i], diag[i], sum);
+    s[0] = pr_add_c(s[0], c0);
 }
 
 template <int W = 4>
 __device__ __forceinline__ void poseidon2_permute(uint64_t s[12], const Poseidon2Tab &tab = c_poseidon2) {
-    poseidon2_external(s, &tab.rcm.v[0]);
+    poseidon2_external(s, tab.rc[0]);
 #pragma unroll 1
-    for (int rnd = 0; rnd < 4; rnd++) {
-        pow7_all<W>(s);
-        poseidon2_external(s, &tab.rcm.v[12 * (rnd + 1)]);
-    }
-    // internal rounds: only lane 0 of their constants is non-zero
+    for (int half = 0; half < 2; half++) {
 #pragma unroll 1
-    for (int rnd = 4; rnd < 26; rnd++) {
-        s[0] = pr_pow7(s[0]);
-        poseidon2_internal(s, &tab.rc.v[12 * (rnd + 1)], tab.diag);
-    }
+        for (int f = 0; f < 4; f++) {
+            pow7_all<W>(s);
+            // after rounds 0-2 and 26-28 the next round's constants, after round 3 those of the
+            // first internal round (lane 0), none after the last
+            poseidon2_external(s, tab.rc[26 * half + f + 1]);
+        }
+        if (half) break;
+        // internal rounds: only lane 0 of their constants is non-zero
 #pragma unroll 1
-    for (int rnd = 26; rnd < 30; rnd++) {
-        pow7_all<W>(s);
-        poseidon2_external(s, rnd < 29 ? &tab.rcm.v[12 * (rnd + 1)] : nullptr);
+        for (int rnd = 4; rnd < 26; rnd++) {
+            s[0] = pr_pow7(s[0]);
+            poseidon2_internal(s, tab.rc[rnd + 1][0], tab.diag);
+        }
+#pragma unroll
+        for (int i = 1; i < 12; i++) s[i] = pr_add_c(s[i], tab.rc[26][i]);
     }
 }
 
@@ -384,50 +493,35 @@ __device__ __forceinline__ void keccak_f1600(uint64_t a[25]) {
 //  * bricks (Feistel type 3): lane i, from 11 down to 1, += (lane i-1)^2 mod p,
 //    the square of lane i-1 before the layer.  zeknox keeps that sum as a
 //    65-bit value for the next concrete layer; here it is taken mod p
-//    (pr_add_c), which is the same field element.
-#define ZK_MONO_ROW constexpr uint32_t row[12] = {ZK_MONOLITH_MDS_ROW_LIST};
-struct MonolithCirc {
-    __host__ __device__ static constexpr int p2(int r, int k) {
-        ZK_MONO_ROW
-        return (int)(row[(k - r + 12) % 12] + row[(k + 6 - r + 12) % 12]);
-    }
-    __host__ __device__ static constexpr int q2(int r, int k) {
-        ZK_MONO_ROW
-        return (int)row[(k - r + 12) % 12] - (int)row[(k + 6 - r + 12) % 12];
+//    (pr_sqr_add), which is the same field element.
+struct MonolithMds {
+    __host__ __device__ static constexpr int c(int j) {
+        constexpr uint32_t row[12] = {ZK_MONOLITH_MDS_ROW_LIST};
+        return (int)row[j];
     }
     __host__ __device__ static constexpr int d0() { return 0; }
 };
-#undef ZK_MONO_ROW
 
-// Accumulator starting values of the 7 concrete layers ("to integers" form:
-// 2^52 + the 32-bit halves of (rc - kMagicAdj) mod p).
+// Accumulator starting values of the 7 concrete layers.
 struct MonolithTab {
-    double k[7][2][12];
+    uint64_t k[7][2][12];
 };
 constexpr MonolithTab make_monolith_tab() {
     MonolithTab t{};
     constexpr uint64_t rc[84] = {ZK_MONOLITH_RC_LIST};
     for (int rnd = 0; rnd < 7; rnd++)
         for (int r = 0; r < 12; r++) {
-            const uint64_t m = cx_sub_mod(cx_canon(rc[12 * rnd + r]), kMagicAdj);
-            t.k[rnd][0][r] = kMagic + (double)(m & 0xffffffffull);
-            t.k[rnd][1][r] = kMagic + (double)(m >> 32);
+            const KPair k = make_kpair(rc[12 * rnd + r], Circ<MonolithMds>::offset<1>(r), kFullBias);
+            t.k[rnd][0][r] = k.lo;
+            t.k[rnd][1][r] = k.hi;
         }
     return t;
 }
 __constant__ MonolithTab c_monolith = make_monolith_tab();
 __device__ MonolithTab g_monolith = make_monolith_tab();
 
-__device__ __forceinline__ void monolith_concrete(uint64_t s[12], const double (*k)[12]) {
-    double a[12], lo[12], hi[12];
-#pragma unroll
-    for (int i = 0; i < 12; i++) a[i] = magic_in((uint32_t)s[i]);
-    circ12_half<MonolithCirc>(a, lo, k[0]);
-#pragma unroll
-    for (int i = 0; i < 12; i++) a[i] = magic_in((uint32_t)(s[i] >> 32));
-    circ12_half<MonolithCirc>(a, hi, k[1]);
-#pragma unroll
-    for (int r = 0; r < 12; r++) s[r] = pr_reduce_split_nc(magic_out(lo[r]), magic_out(hi[r]));
+__device__ __forceinline__ void monolith_concrete(uint64_t s[12], const uint64_t (*k)[12]) {
+    circ_layer<MonolithMds>(s, k);
 #pragma unroll
     for (int r = 0; r < 4; r++) s[r] = gl_canon(s[r]);
 }
@@ -450,7 +544,7 @@ __device__ __forceinline__ void monolith_permute(uint64_t s[12], const MonolithT
         for (int i = 0; i < 4; i++)
             s[i] = ((uint64_t)monolith_bar32((uint32_t)(s[i] >> 32)) << 32) | monolith_bar32((uint32_t)s[i]);
 #pragma unroll
-        for (int i = 11; i > 0; i--) s[i] = pr_add_c(s[i], gl_mul(s[i - 1], s[i - 1]));
+        for (int i = 11; i > 0; i--) s[i] = pr_sqr_add(s[i - 1], s[i]);
         monolith_concrete(s, tab.k[rnd]);
     }
 }
@@ -822,49 +916,96 @@ __device__ __forceinline__ void hash_two(const uint64_t *l, const uint64_t *r, u
 // For trees with too few leaves to fill the GPU one thread per hash, but
 // enough that six threads per hash would be issue-bound: the permutation is
 // split over the two threads of a lane pair (lanes 2k, 2k + 1; sixteen hashes
-// per warp, no idle lanes).  Thread h owns state lanes 6h .. 6h + 5.  Each
-// round: the S-box on the owned lanes (lane 0 only, on thread 0, in partial
-// rounds); then the MDS with the 32-bit halves split between the pair (thread
-// 0 takes the low halves of all 12 lanes, thread 1 the high halves: six
-// 32-bit shuffles bring the partner's halves), the half-vector layer in FP64
-// as in the one-thread path, and six 64-bit shuffles that hand each thread
-// the other half of its own lanes' outputs.  The total work is about that
-// of one thread per hash, spread over twice the threads.
+// per warp, no idle lanes).  Thread h owns state lanes 6h .. 6h + 5 and
+// computes half h of every layer's outputs: six 32-bit shuffles bring the
+// partner's input halves, and six 64-bit shuffles hand each thread the other
+// half of its own lanes' outputs.  In a pair of partial rounds lane 0's first
+// S-box runs on thread 0 and its second one, after an exchange of the halves
+// of y0, on both threads.
 __device__ __forceinline__ uint32_t shfl_xor32(uint32_t v) { return (uint32_t)__shfl_xor_sync(0xffffffffu, (int)v, 1); }
 __device__ __forceinline__ double shfl_xor_d(double v) { return __shfl_xor_sync(0xffffffffu, v, 1); }
+
+// Half h of the state's lanes as sums and differences of lanes i and i + 6.
+__device__ __forceinline__ void duo_inputs(const uint64_t s[6], uint32_t h, double u[6], double w[6]) {
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        const uint32_t lo = (uint32_t)s[i], hi = (uint32_t)(s[i] >> 32);
+        const uint32_t got = shfl_xor32(h ? lo : hi);  // the partner wants the half it computes
+        const uint32_t mine = h ? hi : lo;
+        const uint32_t a = h ? got : mine, b = h ? mine : got;  // lanes 0-5 are thread 0's, 6-11 thread 1's
+        u[i] = sum_dbl(a, b);
+        w[i] = diff_dbl(a, b);
+    }
+}
+// Thread 0 keeps the low outputs of lanes 0-5 and receives their high outputs;
+// thread 1 keeps the high outputs of lanes 6-11 and receives their low outputs.
+__device__ __forceinline__ void duo_outputs(uint64_t s[6], uint32_t h, const double o[12]) {
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        const double got = shfl_xor_d(h ? o[i] : o[i + 6]);
+        const double lo = h ? got : o[i], hi = h ? o[i + 6] : got;
+        s[i] = pr_reduce_split(dbl_int(lo), dbl_int(hi));
+    }
+}
+template <int N>
+__device__ __forceinline__ void duo_rows(const double u[6], const double w[6], double o[12], const uint64_t *k) {
+    using C = PoseidonCirc;
+#pragma unroll
+    for (int r = 0; r < 6; r++) {
+        double pa = (double)C::p<N>(r, 5) * u[5], qa = (double)C::q<N>(r, 5) * w[5];
+#pragma unroll
+        for (int c = 4; c >= 0; c--) {
+            pa = fma((double)C::p<N>(r, c), u[c], pa);
+            qa = fma((double)C::q<N>(r, c), w[c], qa);
+        }
+        o[r] = fma(0.5, pa + qa, int_dbl(k[r]));
+        o[r + 6] = fma(0.5, pa - qa, int_dbl(k[r + 6]));
+    }
+}
 
 // s: lanes 6h .. 6h + 5 (partially reduced, in and out).  Every lane of the
 // warp must call this (shuffles over the full warp).
 __device__ __forceinline__ void poseidon_permute_duo(uint64_t s[6], uint32_t h, const PoseidonTab &tab) {
+    using C = PoseidonCirc;
+    constexpr double d0 = (double)PoseidonMds::d0();
 #pragma unroll
     for (int i = 0; i < 6; i++) s[i] = pr_add_c(s[i], tab.rc0[6 * h + i]);
 #pragma unroll 1
-    for (int rnd = 0; rnd < 30; rnd++) {
-        if (rnd < 4 || rnd >= 26) {
+    for (int half = 0; half < 2; half++) {
+#pragma unroll 1
+        for (int f = 0; f < 4; f++) {
 #pragma unroll
             for (int i = 0; i < 6; i++) s[i] = pr_pow7(s[i]);
-        } else if (h == 0) {
-            s[0] = pr_pow7(s[0]);
+            double u[6], w[6], o[12];
+            duo_inputs(s, h, u, w);
+            duo_rows<1>(u, w, o, tab.full[4 * half + f][h]);
+            // x0 is (u + w - 2^32) / 2; both are exact
+            o[0] = fma(0.5 * d0, u[0] + (w[0] - int_dbl(1ull << 32)), o[0]);
+            duo_outputs(s, h, o);
         }
-        // Half h of all 12 lanes: own lanes directly, the partner's through a shuffle.
-        double a[12], o[12];
+        if (half) break;
+#pragma unroll 1
+        for (int q = 0; q < 11; q++) {
+            if (h == 0) s[0] = pr_pow7(s[0]);
+            double u[6], w[6], o[12];
+            duo_inputs(s, h, u, w);
+            const double x0 = 0.5 * (u[0] + (w[0] - int_dbl(1ull << 32)));
+            double pa = 0, qa = 0;
 #pragma unroll
-        for (int i = 0; i < 6; i++) {
-            const uint32_t lo = (uint32_t)s[i], hi = (uint32_t)(s[i] >> 32);
-            const uint32_t got = shfl_xor32(h ? lo : hi);  // the partner wants the half it computes
-            const uint32_t mine = h ? hi : lo;
-            a[i] = magic_in(h ? got : mine);       // lanes 0-5: thread 0's own, thread 1's received
-            a[i + 6] = magic_in(h ? mine : got);   // lanes 6-11: thread 1's own, thread 0's received
-        }
-        poseidon_mds_half(a, o, tab.mdsk.v[rnd][h]);
-        // Thread 0 keeps the low outputs of lanes 0-5 and receives their high
-        // outputs; thread 1 keeps the high outputs of lanes 6-11 and receives
-        // their low outputs.
+            for (int i = 5; i >= 0; i--) {
+                pa = fma((double)C::p<1>(0, i), u[i], pa);
+                qa = fma((double)C::q<1>(0, i), w[i], qa);
+            }
+            const double y0 = fma(0.5, pa + qa, fma(d0, x0, int_dbl(tab.mid[q][h])));
+            const double other = shfl_xor_d(y0);
+            const uint64_t y = pr_pow7(pr_reduce_split(dbl_int(h ? other : y0), dbl_int(h ? y0 : other)));
+            const double yp = word_dbl(h ? (uint32_t)(y >> 32) : (uint32_t)y);
+            const double g = fma(d0, x0, yp - y0);
+            duo_rows<2>(u, w, o, tab.pair[q][h]);
 #pragma unroll
-        for (int i = 0; i < 6; i++) {
-            const double got = shfl_xor_d(h ? o[i] : o[i + 6]);
-            const double lo = h ? got : o[i], hi = h ? o[i + 6] : got;
-            s[i] = pr_reduce_split_nc(magic_out(lo), magic_out(hi));
+            for (int r = 0; r < 12; r++) o[r] = fma((double)C::at(-r), g, o[r]);
+            o[0] = fma(d0, yp, o[0]);
+            duo_outputs(s, h, o);
         }
     }
 }
@@ -900,13 +1041,14 @@ __device__ __forceinline__ void poseidon_hash_one_duo(const uint64_t *in, uint32
 // For the latency-bound parts (narrow tree levels, small trees) one
 // permutation is spread over a group of six consecutive lanes of a warp
 // (five groups per warp; lanes 30 and 31 compute on dummy data).  Group
-// thread t owns lanes t and t + 6.  Each round: the S-box on the owned lanes
-// (lane 0 only, on thread 0, in partial rounds), an all-gather of the 12
-// lanes by shuffles (every shuffle reads one thread of the group, so all
-// threads get the lanes in natural order), then thread t computes the MDS
-// row pair (t, t + 6) of the split above: rows of A + B and A - B held in
-// registers.  About a third of the single-thread path's instructions per
-// thread, so about a third of its latency.
+// thread t owns lanes t and t + 6.  Each round or pair of partial rounds: an
+// all-gather of the 12 lanes by shuffles (every shuffle reads one thread of
+// the group, so all threads get the lanes in natural order), then thread t
+// computes the row pair (t, t + 6) of the layer, its rows of A + B and A - B
+// held in registers.  Full rounds apply the S-box to the owned lanes before
+// the gather; in a pair every thread runs both of lane 0's S-boxes itself, so
+// that a pair needs one gather and no further exchange, and the other lanes'
+// shuffles hide behind the first S-box.
 struct HexLanes {
     uint32_t t;     // thread within the group, 0..5 (lanes 30, 31: 0..1 of a dummy group)
     uint32_t base;  // warp lane of the group's thread 0
@@ -920,18 +1062,24 @@ struct HexLanes {
     __device__ __forceinline__ bool real() const { return (threadIdx.x & 31) < 30; }
     __device__ __forceinline__ uint32_t group_in_warp() const { return base / 6; }
 };
-// Poseidon's group: its MDS rows in registers.  (The table argument gives the
-// Poseidon and Poseidon2 group forms one constructor signature.)
+// Poseidon's group: its rows in registers.
 struct HexGroup : HexLanes {
-    double p2[6], q2[6];  // row t of A + B and A - B (with the diagonal term on row 0)
-    double fix6;          // -2 d on thread 0 (lane 6 must not get the diagonal), else 0
-    __device__ __forceinline__ explicit HexGroup(const PoseidonTab &) : HexLanes() {
+    double p1[6], q1[6];  // row t of A + B and A - B
+    double p2[6], q2[6];  // row t of their squares
+    double c0, c6;        // C e0 at rows t and t + 6
+    double d0;            // the diagonal term on thread 0, else 0
+    __device__ __forceinline__ explicit HexGroup(const PoseidonTab &tab) : HexLanes() {
+        const double *row = tab.rows[t];
 #pragma unroll
         for (int k = 0; k < 6; k++) {
-            p2[k] = (double)mds_p2((int)t, k);
-            q2[k] = (double)mds_q2((int)t, k);
+            p1[k] = row[k];
+            q1[k] = row[6 + k];
+            p2[k] = row[12 + k];
+            q2[k] = row[18 + k];
         }
-        fix6 = t == 0 ? -2.0 * (double)mds_diag0() : 0.0;
+        c0 = row[24];
+        c6 = row[25];
+        d0 = t == 0 ? (double)PoseidonMds::d0() : 0.0;
     }
 };
 
@@ -943,45 +1091,70 @@ __device__ __forceinline__ uint64_t shfl64(uint64_t v, uint32_t src) {
 // Every lane of the warp must call this (shuffles over the full warp).
 __device__ __forceinline__ void poseidon_permute_hex(uint64_t &o0, uint64_t &o1, const HexGroup &g,
                                                      const PoseidonTab &tab) {
+    using C = PoseidonCirc;
+    constexpr double d0 = (double)PoseidonMds::d0();
     o0 = pr_add_c(o0, tab.rc0[g.t]);
     o1 = pr_add_c(o1, tab.rc0[g.t + 6]);
 #pragma unroll 1
-    for (int rnd = 0; rnd < 30; rnd++) {
-        if (rnd < 4 || rnd >= 26) {
+    for (int half = 0; half < 2; half++) {
+#pragma unroll 1
+        for (int f = 0; f < 4; f++) {
             o0 = pr_pow7(o0);
             o1 = pr_pow7(o1);
-        } else {
-            const uint64_t y = pr_pow7(o0);
-            if (g.t == 0) o0 = y;
-        }
-        uint64_t x[12];
+            uint64_t x[12];
 #pragma unroll
-        for (int i = 0; i < 12; i++) x[i] = shfl64(i < 6 ? o0 : o1, g.base + (i % 6));
-        double first[2], second[2];
+            for (int i = 0; i < 12; i++) x[i] = shfl64(i < 6 ? o0 : o1, g.base + (i % 6));
+            double first[2], second[2];
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            double u[6], w[6], x6 = 0.0;
+            for (int h = 0; h < 2; h++) {
+                double pa = 0, qa = 0;
 #pragma unroll
-            for (int i = 0; i < 6; i++) {
-                const double a = magic_in(h ? (uint32_t)(x[i] >> 32) : (uint32_t)x[i]);
-                const double b = magic_in(h ? (uint32_t)(x[i + 6] >> 32) : (uint32_t)x[i + 6]);
-                const double tb = b - kMagic;
-                if (i == 0) x6 = tb;
-                w[i] = a - b;
-                u[i] = fma(2.0, tb, w[i]);
+                for (int k = 0; k < 6; k++) {
+                    pa = fma(g.p1[k], sum_dbl(half_of(x[k], h), half_of(x[k + 6], h)), pa);
+                    qa = fma(g.q1[k], diff_dbl(half_of(x[k], h), half_of(x[k + 6], h)), qa);
+                }
+                first[h] = fma(0.5, pa + qa,
+                               fma(g.d0, word_dbl(half_of(x[0], h)), int_dbl(tab.full[4 * half + f][h][g.t])));
+                second[h] = fma(0.5, pa - qa, int_dbl(tab.full[4 * half + f][h][g.t + 6]));
             }
-            double pa = g.p2[0] * u[0], qa = g.q2[0] * w[0];
-#pragma unroll
-            for (int k = 1; k < 6; k++) {
-                pa = fma(g.p2[k], u[k], pa);
-                qa = fma(g.q2[k], w[k], qa);
-            }
-            const double d = fma(g.fix6, x6, pa - qa);
-            first[h] = fma(0.5, pa + qa, tab.mdsk.v[rnd][h][g.t]);
-            second[h] = fma(0.5, d, tab.mdsk.v[rnd][h][g.t + 6]);
+            o0 = pr_reduce_split(dbl_int(first[0]), dbl_int(first[1]));
+            o1 = pr_reduce_split(dbl_int(second[0]), dbl_int(second[1]));
         }
-        o0 = pr_reduce_split_nc(magic_out(first[0]), magic_out(first[1]));
-        o1 = pr_reduce_split_nc(magic_out(second[0]), magic_out(second[1]));
+        if (half) break;
+#pragma unroll 1
+        for (int q = 0; q < 11; q++) {
+            uint64_t x[12];
+#pragma unroll
+            for (int i = 0; i < 12; i++) x[i] = shfl64(i < 6 ? o0 : o1, g.base + (i % 6));
+            x[0] = pr_pow7(x[0]);
+            double first[2], second[2], y0[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                double pa = 0, qa = 0, pb = 0, qb = 0;
+#pragma unroll
+                for (int k = 5; k >= 0; k--) {
+                    const double u = sum_dbl(half_of(x[k], h), half_of(x[k + 6], h));
+                    const double w = diff_dbl(half_of(x[k], h), half_of(x[k + 6], h));
+                    pa = fma((double)C::p<1>(0, k), u, pa);
+                    qa = fma((double)C::q<1>(0, k), w, qa);
+                    pb = fma(g.p2[k], u, pb);
+                    qb = fma(g.q2[k], w, qb);
+                }
+                y0[h] = fma(0.5, pa + qa, fma(d0, word_dbl(half_of(x[0], h)), int_dbl(tab.mid[q][h])));
+                first[h] = fma(0.5, pb + qb, int_dbl(tab.pair[q][h][g.t]));
+                second[h] = fma(0.5, pb - qb, int_dbl(tab.pair[q][h][g.t + 6]));
+            }
+            const uint64_t y = pr_pow7(pr_reduce_split(dbl_int(y0[0]), dbl_int(y0[1])));
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const double yp = word_dbl(half_of(y, h));
+                const double e = fma(d0, word_dbl(half_of(x[0], h)), yp - y0[h]);
+                first[h] = fma(g.d0, yp, fma(g.c0, e, first[h]));
+                second[h] = fma(g.c6, e, second[h]);
+            }
+            o0 = pr_reduce_split(dbl_int(first[0]), dbl_int(first[1]));
+            o1 = pr_reduce_split(dbl_int(second[0]), dbl_int(second[1]));
+        }
     }
 }
 
@@ -994,7 +1167,7 @@ __device__ __forceinline__ void poseidon_permute_hex(uint64_t &o0, uint64_t &o1,
 // column (t + 2) % 4, so thread t needs only m = M4[t % 4]: lane t takes
 // x_(4b + d) with m[d], lane t + 6 with m[(d + 2) % 4], and each lane weighs
 // the three block sums by w in {1, 2}.  As in the one-thread layer, each
-// 32-bit half runs in exact FP64 (every sum below 2^39), offset by 2^52.
+// 32-bit half runs in exact FP64 (every sum below 2^39).
 //
 // Internal layer (x_i <- x_i D_i + sum_j x_j + c_i): each thread adds its
 // two lanes exactly (65 bits), the group all-gathers the six partial sums
@@ -1002,7 +1175,7 @@ __device__ __forceinline__ void poseidon_permute_hex(uint64_t &o0, uint64_t &o1,
 struct HexGroup2 : HexLanes {
     double m[4];          // row t % 4 of M4
     double w0[3], w1[3];  // block weights of lanes t and t + 6
-    uint64_t d0, d1;      // internal diagonal of lanes t and t + 6
+    uint64_t d0, d1;      // internal diagonal of lanes t and t + 6, times 2^64
     __device__ __forceinline__ explicit HexGroup2(const Poseidon2Tab &tab) : HexLanes() {
         // M4 rows 0 and 1; rows 2 and 3 are these rotated by two columns.
         const uint32_t c = t & 3, r = c & 1, rot = c & 2;
@@ -1023,10 +1196,9 @@ struct HexGroup2 : HexLanes {
     }
 };
 
-// External layer on a group, plus the constants cm (adjusted for the magic
-// offsets; nullptr: none).
+// External layer on a group, plus the constants c.
 __device__ __forceinline__ void poseidon2_external_hex(uint64_t &o0, uint64_t &o1, const HexGroup2 &g,
-                                                       const uint64_t *cm) {
+                                                       const uint64_t *c) {
     uint64_t x[12];
 #pragma unroll
     for (int i = 0; i < 12; i++) x[i] = shfl64(i < 6 ? o0 : o1, g.base + (i % 6));
@@ -1035,8 +1207,8 @@ __device__ __forceinline__ void poseidon2_external_hex(uint64_t &o0, uint64_t &o
     for (int h = 0; h < 2; h++) {
         double v[12];
 #pragma unroll
-        for (int i = 0; i < 12; i++) v[i] = magic_in(h ? (uint32_t)(x[i] >> 32) : (uint32_t)x[i]) - kMagic;
-        double a0 = kMagic, a1 = kMagic;
+        for (int i = 0; i < 12; i++) v[i] = word_dbl(half_of(x[i], h));
+        double a0 = 0, a1 = 0;
 #pragma unroll
         for (int b = 0; b < 3; b++) {
             double y0 = g.m[0] * v[4 * b], y1 = g.m[2] * v[4 * b];
@@ -1051,13 +1223,12 @@ __device__ __forceinline__ void poseidon2_external_hex(uint64_t &o0, uint64_t &o
         first[h] = a0;
         second[h] = a1;
     }
-    o0 = pr_reduce_split(magic_out(first[0]), magic_out(first[1]), cm ? cm[g.t] : kMagicNeg);
-    o1 = pr_reduce_split(magic_out(second[0]), magic_out(second[1]), cm ? cm[g.t + 6] : kMagicNeg);
+    o0 = pr_reduce_split_add(dbl_int(first[0]), dbl_int(first[1]), c[g.t]);
+    o1 = pr_reduce_split_add(dbl_int(second[0]), dbl_int(second[1]), c[g.t + 6]);
 }
 
-// Internal layer on a group, plus the next round's constants c (unadjusted).
-__device__ __forceinline__ void poseidon2_internal_hex(uint64_t &o0, uint64_t &o1, const HexGroup2 &g,
-                                                       const uint64_t *c) {
+// Internal layer on a group (poseidon2_internal without the constant).
+__device__ __forceinline__ void poseidon2_internal_hex(uint64_t &o0, uint64_t &o1, const HexGroup2 &g) {
     uint32_t p0, p1, p2;
     asm("add.cc.u32 %0, %3, %5;\n\t"
         "addc.cc.u32 %1, %4, %6;\n\t"
@@ -1077,44 +1248,32 @@ __device__ __forceinline__ void poseidon2_internal_hex(uint64_t &o0, uint64_t &o
             : "+r"(s0), "+r"(s1), "+r"(s2)
             : "r"(q0), "r"(q1), "r"(q2));
     }
-    uint64_t lane[2] = {o0, o1};
-    const uint64_t cc[2] = {c[g.t], c[g.t + 6]};
-    const uint64_t dd[2] = {g.d0, g.d1};
-#pragma unroll
-    for (int j = 0; j < 2; j++) {
-        uint32_t c0, c1, c2;
-        asm("add.cc.u32 %0, %3, %6;\n\t"
-            "addc.cc.u32 %1, %4, %7;\n\t"
-            "addc.u32 %2, %5, 0;"
-            : "=r"(c0), "=r"(c1), "=r"(c2)
-            : "r"(s0), "r"(s1), "r"(s2), "r"((uint32_t)cc[j]), "r"((uint32_t)(cc[j] >> 32)));
-        lane[j] = pr_mul_add(lane[j], dd[j], ((uint64_t)c1 << 32) | c0, c2);
-    }
-    o0 = lane[0];
-    o1 = lane[1];
+    const uint64_t sum = poseidon2_sum_mont(s0, s1, s2);
+    o0 = poseidon2_lane(o0, g.d0, sum);
+    o1 = poseidon2_lane(o1, g.d1, sum);
 }
 
 // The rounds of poseidon2_permute on a group.
 __device__ __forceinline__ void poseidon2_permute_hex(uint64_t &o0, uint64_t &o1, const HexGroup2 &g,
                                                       const Poseidon2Tab &tab) {
-    poseidon2_external_hex(o0, o1, g, &tab.rcm.v[0]);
+    poseidon2_external_hex(o0, o1, g, tab.rc[0]);
 #pragma unroll 1
-    for (int rnd = 0; rnd < 4; rnd++) {
-        o0 = pr_pow7(o0);
-        o1 = pr_pow7(o1);
-        poseidon2_external_hex(o0, o1, g, &tab.rcm.v[12 * (rnd + 1)]);
-    }
+    for (int half = 0; half < 2; half++) {
 #pragma unroll 1
-    for (int rnd = 4; rnd < 26; rnd++) {
-        const uint64_t y = pr_pow7(o0);
-        if (g.t == 0) o0 = y;
-        poseidon2_internal_hex(o0, o1, g, &tab.rc.v[12 * (rnd + 1)]);
-    }
+        for (int f = 0; f < 4; f++) {
+            o0 = pr_pow7(o0);
+            o1 = pr_pow7(o1);
+            poseidon2_external_hex(o0, o1, g, tab.rc[26 * half + f + 1]);
+        }
+        if (half) break;
 #pragma unroll 1
-    for (int rnd = 26; rnd < 30; rnd++) {
-        o0 = pr_pow7(o0);
-        o1 = pr_pow7(o1);
-        poseidon2_external_hex(o0, o1, g, rnd < 29 ? &tab.rcm.v[12 * (rnd + 1)] : nullptr);
+        for (int rnd = 4; rnd < 26; rnd++) {
+            const uint64_t y = pr_pow7(o0);
+            if (g.t == 0) o0 = y;
+            poseidon2_internal_hex(o0, o1, g);
+            o0 = pr_add_c(o0, tab.rc[rnd + 1][g.t]);  // only lane 0's is non-zero before round 26
+            if (rnd == 25) o1 = pr_add_c(o1, tab.rc[26][g.t + 6]);
+        }
     }
 }
 

@@ -92,7 +92,8 @@ ZK_PROBE_OP(probe_mul2_24, a = gl_mul2_24(a); b = b ^ a)
 ZK_PROBE_OP(probe_mul2_48, a = gl_mul2_48(a); b = b ^ a)
 ZK_PROBE_OP(probe_mul2_72, a = gl_mul2_72(a); b = b ^ a)
 ZK_PROBE_OP(probe_pr_mul, a = pr_mul(a, b); b = b ^ a)
-ZK_PROBE_OP(probe_pr_sqr, a = pr_sqr(a); b = b ^ a)
+ZK_PROBE_OP(probe_mont_mul, a = mont_mul(a, b); b = b ^ a)
+ZK_PROBE_OP(probe_mont_sqr, a = mont_sqr(a); b = b ^ a)
 ZK_PROBE_OP(probe_pr_pow7, a = pr_pow7(a); b = b ^ a)
 #undef ZK_PROBE_OP
 
@@ -126,7 +127,7 @@ extern "C" __attribute__((visibility("default"))) int zk_probe_field_ops(int ite
     if (cudaMalloc(&out, 32 * sizeof(uint64_t)) != cudaSuccess) return -2;
     void (*ops[])(uint64_t *, uint64_t, uint64_t, int) = {
         probe_base, probe_nt_add, probe_nt_sub, probe_nt_mul, probe_mul2_24, probe_mul2_48, probe_mul2_72,
-        probe_pr_mul, probe_pr_sqr, probe_pr_pow7, probe_dft8_base, probe_dft8};
+        probe_pr_mul, probe_mont_mul, probe_mont_sqr, probe_pr_pow7, probe_dft8_base, probe_dft8};
     for (auto k : ops) k<<<1, 32>>>(out, 0x123456789abcdefull, 0xfedcba9876543210ull, iters);
     cudaError_t e = cudaDeviceSynchronize();
     cudaFree(out);
