@@ -1,4 +1,4 @@
-"""The hash kernels' arithmetic (gl64.cuh, hash.cuh) replayed on the CPU with
+"""The hash kernels' and the NTT's arithmetic (gl64.cuh, hash.cuh, ntt_field.cuh) replayed on the CPU with
 PTX's carry semantics: the Montgomery reduction, x^7 from four Montgomery
 products, the folds that end the linear layers, Poseidon2's diagonal lane, and
 the two-rounds-at-once form of Poseidon's partial rounds with the bounds that
@@ -111,6 +111,15 @@ def test_poseidon2_diagonal_lane():
             v = x * (d * R % P) + s
             assert v < 2**128
             assert mont_reduce(v) % P == (x * d + z) % P
+
+
+def test_ntt_power_of_two_products():
+    """ntt_field.cuh: x 2^24 as a fold, -x 2^48 as a Montgomery reduction of x 2^16; canonical results."""
+    for x in values(3000, 6):
+        x %= P
+        v = x << 24
+        assert pr_fold(v & M32, v >> 32 & M32, v >> 64) == x * 2**24 % P
+        assert mont_reduce(x << 16) == -x * 2**48 % P
 
 
 def poseidon_constants():

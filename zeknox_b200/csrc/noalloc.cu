@@ -57,9 +57,9 @@ static __device__ __align__(256) uint64_t g_noalloc[kTotalElems];
 std::mutex g_mu;
 uint64_t *g_base[kMaxDevices] = {};
 
-// b^e for e < 2^bits by square-and-multiply.
+// b^e times 2^64 (the form of every power table) by square-and-multiply.
 __device__ uint64_t dev_pow(uint64_t b, uint64_t e) {
-    uint64_t r = 1;
+    uint64_t r = ZK_EPS;
     while (e) {
         if (e & 1) r = zk::gl_mul(r, b);
         b = zk::gl_mul(b, b);

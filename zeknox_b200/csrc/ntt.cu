@@ -65,8 +65,8 @@ struct PassArgs {
     const uint64_t *post_lo, *post_hi;  // coset powers (null: none)
     const uint64_t *post_full;
     uint32_t post_h;
-    uint64_t scale;     // 1 = none
-    // twiddles
+    uint64_t scale;     // times 2^64 (nt_mul); 1 = none
+    // twiddles (these and the coset powers are stored times 2^64, as nt_mul takes them)
     const uint64_t *tw_lo, *tw_hi;  // omega_N powers (two-level)
     const uint64_t *tw_full;        // omega_N^e for every e < N (null above 2^20 points)
     uint32_t tw_h;
@@ -139,7 +139,7 @@ __device__ __forceinline__ void smem_dif(uint64_t *sm, const uint64_t *tw, uint3
             const uint64_t x0 = sm[e0 * tp + t], x1 = sm[(e0 + 1) * tp + t], x2 = sm[(e0 + 2) * tp + t],
                            x3 = sm[(e0 + 3) * tp + t];
             const uint64_t a0 = nt_add(x0, x2), a2 = nt_sub(x0, x2), a1 = nt_add(x1, x3);
-            const uint64_t a3 = inv ? gl_mul2_48(nt_sub(x3, x1)) : gl_mul2_48(nt_sub(x1, x3));
+            const uint64_t a3 = inv ? gl_mul2_48_neg(nt_sub(x1, x3)) : gl_mul2_48_neg(nt_sub(x3, x1));
             sm[e0 * tp + t] = nt_add(a0, a1);
             sm[(e0 + 1) * tp + t] = nt_sub(a0, a1);
             sm[(e0 + 2) * tp + t] = nt_add(a2, a3);
@@ -204,7 +204,7 @@ __device__ __forceinline__ void smem_dif_fixed(uint64_t *sm, const uint64_t *tw)
                     uint64_t *b = sm + ((u >> LG_T) << 2) * TP + (u & (T - 1));
                     const uint64_t x0 = b[0], x1 = b[TP], x2 = b[2 * TP], x3 = b[3 * TP];
                     const uint64_t a0 = nt_add(x0, x2), a2 = nt_sub(x0, x2), a1 = nt_add(x1, x3);
-                    const uint64_t a3 = INV ? gl_mul2_48(nt_sub(x3, x1)) : gl_mul2_48(nt_sub(x1, x3));
+                    const uint64_t a3 = INV ? gl_mul2_48_neg(nt_sub(x1, x3)) : gl_mul2_48_neg(nt_sub(x3, x1));
                     b[0] = nt_add(a0, a1);
                     b[TP] = nt_sub(a0, a1);
                     b[2 * TP] = nt_add(a2, a3);
@@ -945,7 +945,7 @@ static PassArgs transform_args(const NttJob &j, const PowTable &roots, const uin
     base.tw_full = roots.full;
     base.line_roots = line_roots_dev;
     base.inverse = j.inverse ? 1u : 0u;
-    base.scale = j.scale;
+    base.scale = j.scale == 1 ? 1 : h_mont(j.scale);
     base.batches = (uint32_t)j.batches;
     if (j.pre_coset) {
         base.pre_lo = j.pre_coset->lo();

@@ -89,7 +89,7 @@ ZK_PROBE_OP(probe_nt_add, a = nt_add(a, b); b = b ^ a)
 ZK_PROBE_OP(probe_nt_sub, a = nt_sub(a, b); b = b ^ a)
 ZK_PROBE_OP(probe_nt_mul, a = nt_mul(a, b); b = b ^ a)
 ZK_PROBE_OP(probe_mul2_24, a = gl_mul2_24(a); b = b ^ a)
-ZK_PROBE_OP(probe_mul2_48, a = gl_mul2_48(a); b = b ^ a)
+ZK_PROBE_OP(probe_mul2_48, a = gl_mul2_48_neg(a); b = b ^ a)
 ZK_PROBE_OP(probe_mul2_72, a = gl_mul2_72(a); b = b ^ a)
 ZK_PROBE_OP(probe_pr_mul, a = pr_mul(a, b); b = b ^ a)
 ZK_PROBE_OP(probe_mont_mul, a = mont_mul(a, b); b = b ^ a)

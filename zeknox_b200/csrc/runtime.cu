@@ -56,15 +56,15 @@ PowTable make_pow_table(uint64_t base, unsigned bits) {
     t.h = (bits + 1) / 2;
     const uint64_t nlo = 1ull << t.h, nhi = 1ull << (bits - t.h);
     std::vector<uint64_t> v(nlo + nhi);
-    uint64_t x = 1;
-    for (uint64_t i = 0; i < nlo; i++, x = h_mul(x, base)) v[i] = x;  // x = base^nlo at exit
-    const uint64_t step = x;
-    uint64_t y = 1;
+    uint64_t x = h_mont(1);
+    for (uint64_t i = 0; i < nlo; i++, x = h_mul(x, base)) v[i] = x;
+    const uint64_t step = h_pow(base, nlo);
+    uint64_t y = h_mont(1);
     for (uint64_t i = 0; i < nhi; i++, y = h_mul(y, step)) v[nlo + i] = y;
     t.dev = upload(v);
     if (bits <= kFullTableMaxLg) {
         std::vector<uint64_t> f(1ull << bits);
-        uint64_t z = 1;
+        uint64_t z = h_mont(1);
         for (auto &e : f) {
             e = z;
             z = h_mul(z, base);
@@ -110,7 +110,7 @@ const uint64_t *line_roots(DeviceCtx &c, bool inv) {
         uint64_t w = h_omega(kLineLgMax);
         if (inv) w = h_inv(w);
         std::vector<uint64_t> v(1u << kLineLgMax);
-        uint64_t x = 1;
+        uint64_t x = h_mont(1);
         for (auto &e : v) {
             e = x;
             x = h_mul(x, w);

@@ -64,10 +64,13 @@ inline uint64_t h_pow(uint64_t a, uint64_t e) {
 inline uint64_t h_inv(uint64_t a) { return h_pow(a, P_HOST - 2); }
 // Primitive 2^lg-th root of unity: 7^((p-1)/2^lg) (zeknox native/ff/gl64_params.hpp:15).
 inline uint64_t h_omega(unsigned lg) { return h_pow(7, (P_HOST - 1) >> lg); }
+// The form of the device tables' values: a 2^64 mod p (a never is 2^-64 there, so never 1).
+inline uint64_t h_mont(uint64_t a) { return h_mul(a, 0xffffffffull); }
 constexpr uint64_t GROUP_GENERATOR = 7;  // native/ff/gl64_params.hpp:12
 
 // Two-level power table of a base b:  b^e = lo[e & (2^h - 1)] * hi[e >> h]
-// for e < 2^bits.  Both halves live in one device allocation.
+// for e < 2^bits.  Both halves live in one device allocation.  Every value is
+// stored times 2^64 (h_mont), the form nt_mul multiplies by.
 struct PowTable {
     uint64_t *dev = nullptr;  // [lo (2^h) | hi (2^(bits-h))]
     uint64_t *full = nullptr; // b^e for every e < 2^bits when bits <= kFullTableMaxLg, else null
