@@ -185,3 +185,68 @@ def test_two_partial_rounds_at_once(seed):
                 acc.append(v)
             out.append(pr_reduce_split_add(*acc) % P)
         assert out == want
+
+
+BN_R = 0x30644E72E131A029B85045B68181585D2833E84879B9709143E1F593F0000001
+MASK = 2**29 - 1
+
+
+def limbs(x):
+    return [x >> (29 * i) & MASK for i in range(9)]
+
+
+def bn_value(v):
+    return sum(a << (29 * i) for i, a in enumerate(v))
+
+
+def bn_mul_sum(terms, addend=(0,) * 9):
+    """(sum of x y) / 2^261 + addend mod r as the kernel's 64-bit columns form it."""
+    ninv = -pow(BN_R, -1, 2**29) % 2**29
+    c = [0] * 9 + list(addend)
+    for x, y in terms:
+        for i in range(9):
+            for j in range(9):
+                c[i + j] += x[i] * y[j]
+    for i in range(9):
+        m = c[i] * ninv & MASK
+        for j, r in enumerate(limbs(BN_R)):
+            c[i + j] += m * r
+        assert max(c) < 2**64
+        c[i + 1] += c[i] >> 29
+    out = []
+    for i in range(9):
+        out.append(c[9 + i] & MASK)
+        if i < 8:
+            c[10 + i] += c[9 + i] >> 29
+        else:
+            assert c[17] <= MASK  # the value is below 2^261
+    assert max(c) < 2**64
+    return out
+
+
+def test_bn254_columns_hold_a_matrix_row():
+    """Five products of full limbs and a reduction fit the columns; results are the field's."""
+    rnd = random.Random(7)
+    top = limbs(BN_R - 1)
+    full = [MASK] * 8 + [(67 * BN_R) >> 232]  # the largest state value of the partial rounds, every other limb full
+    for x, y in [(full, [MASK] * 8 + [top[8]]), (limbs(rnd.randrange(67 * BN_R)), limbs(rnd.randrange(BN_R)))]:
+        got = bn_value(bn_mul_sum([(x, y)] * 5, x))
+        want = 5 * bn_value(x) * bn_value(y) * pow(2**261, -1, BN_R) + bn_value(x)
+        assert got % BN_R == want % BN_R and got < 2**261
+
+
+def test_bn254_partial_round_growth():
+    """Sixty rounds of the lanes' update from the largest first-half outputs stay below 2^260."""
+    rnd = random.Random(8)
+    st = limbs(2 * BN_R - 1)
+    for _ in range(60):
+        st = bn_mul_sum([(limbs(2 * BN_R - 1), limbs(BN_R - 1 - rnd.getrandbits(20)))], st)
+    assert bn_value(st) < 2**260
+    # a full round's S-box of that value: squares below 2^259, the fifth power below 2^256
+    x2 = bn_mul_sum([(st, st)])
+    x4 = bn_mul_sum([(x2, x2)])
+    x5 = bn_mul_sum([(x4, st)], limbs(BN_R - 1))
+    assert bn_value(x2) < 2**259 and bn_value(x5) < 2**256
+    assert bn_mul_sum([], limbs(0)) == [0] * 9
+    # out of Montgomery form the value is at most r
+    assert bn_value(bn_mul_sum([(limbs(2**261 - 1), limbs(1))])) <= BN_R

@@ -6,8 +6,8 @@
 // all subtrees, and a last one the narrow top and the cap: the structure of
 // zeknox's kernels (merkle.cu:215-243).  For Poseidon and Poseidon2, the
 // latency-bound parts (small trees, narrow levels, the top) spread each
-// permutation over six threads (Poseidon also over two) instead (hash.cuh),
-// with thresholds set by measurement.
+// permutation over six threads (Poseidon also over two, Poseidon-BN128 over
+// five) instead (hash.cuh), with thresholds set by measurement.
 // Fusing the lower levels into the leaf kernel (a block folding its tile of
 // leaves through shared memory) measured slower on B200: a block then holds
 // its registers through the serial, mostly idle fold levels, which costs more
@@ -197,6 +197,69 @@ __global__ void __launch_bounds__(224) merkle_top_hex(uint64_t *__restrict__ dig
     }
 }
 
+// Poseidon-BN128 on five threads per hash: six hashes per warp.  A few warps
+// per SM, each with the round tables in shared memory.
+constexpr int kBnThreads = 64;
+constexpr uint64_t kBnPerBlock = 12;
+
+__global__ void __launch_bounds__(kBnThreads) merkle_leaves_bn(const uint64_t *__restrict__ leaves, uint64_t n_leaves,
+                                                               uint32_t leaf_size, uint64_t *__restrict__ out,
+                                                               LeafMap map) {
+    __shared__ BnTab tab;
+    load_tab<kPoseidonBN128>(tab);
+    const BnLanes g;
+    const uint64_t first = ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5) * 6;
+    if (first >= n_leaves) return;  // whole warp
+    const uint64_t i = first + g.group_in_warp();
+    const bool active = g.real() && i < n_leaves;
+    const uint64_t ii = active ? i : 0;
+    bn_hash_one_group(leaves + ii * leaf_size, leaf_size, out + 4 * map.slot(ii), active, g, tab);
+    pdl_release();
+}
+__global__ void __launch_bounds__(kBnThreads) merkle_level_bn(uint64_t *__restrict__ digests, uint32_t lg_w,
+                                                              uint64_t n_caps, uint64_t ds) {
+    __shared__ BnTab tab;
+    load_tab<kPoseidonBN128>(tab);
+    const BnLanes g;
+    const uint64_t w = 1ull << lg_w;
+    const uint64_t first = ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5) * 6;
+    if (first >= (n_caps << lg_w)) return;  // whole warp
+    const uint64_t tid = first + g.group_in_warp();
+    const bool active = g.real() && tid < (n_caps << lg_w);
+    const uint64_t tt = active ? tid : 0;
+    const uint64_t sub = tt >> lg_w, i = (w - 2) + (tt & (w - 1));
+    uint64_t *base = digests + 4 * sub * ds;
+    pdl_wait();
+    bn_hash_two_group(base + 4 * (2 * i + 2), base + 4 * (2 * i + 3), base + 4 * i, active, g, tab);
+    pdl_release();
+}
+// One block per subtree: levels of width w_top (<= 16) .. 1, then the cap.
+__global__ void __launch_bounds__(96) merkle_top_bn(uint64_t *__restrict__ digests, uint64_t *__restrict__ cap,
+                                                    uint64_t ds, uint32_t w_top) {
+    __shared__ BnTab tab;
+    load_tab<kPoseidonBN128>(tab);
+    const BnLanes g;
+    const uint64_t sub = blockIdx.x;
+    uint64_t *base = digests + 4 * sub * ds;
+    const uint32_t node = (threadIdx.x >> 5) * 6 + g.group_in_warp();
+    pdl_wait();
+    for (uint32_t w = w_top; w >= 1; w >>= 1) {
+        if ((threadIdx.x >> 5) * 6 < w) {  // warps with at least one node of this level
+            const bool active = g.real() && node < w;
+            const uint32_t i = active ? node : 0;
+            const uint64_t *c = base + 4 * (2 * w - 2 + 2 * i);  // children 2i, 2i+1 of the level of width 2w
+            uint64_t *o = w >= 2 ? base + 4 * (w - 2 + i) : cap + 4 * sub;
+            bn_hash_two_group(c, c + 4, o, active, g, tab);
+        }
+        __syncthreads();
+    }
+}
+inline unsigned bn_blocks(uint64_t hashes) {
+    const uint64_t b = (hashes + kBnPerBlock - 1) / kBnPerBlock;
+    require(b < (1ull << 31), "Merkle launch too large");
+    return (unsigned)(b ? b : 1);
+}
+
 inline unsigned hex_blocks(uint64_t hashes) {
     const uint64_t b = (hashes + kHexPerBlock - 1) / kHexPerBlock;
     require(b < (1ull << 31), "Merkle launch too large");
@@ -211,13 +274,13 @@ inline unsigned blocks_for(uint64_t n, unsigned tpb) {
 
 
 // Threads per Poseidon hash for a tree's leaves: 6 (HexGroup), 2 (lane
-// pairs) or 1.  Static thresholds, measured on trees of 135-word leaves:
-// whole trees, six- vs one-threaded leaves, 8192 leaves 0.48 vs 0.65 ms,
-// 16384 leaves 0.80 vs 0.68 ms, 32768 leaves 1.43 vs 0.87 ms; two threads per
-// hash win between the two, 16384 leaves 0.59 ms (4096: 0.47, 8192: 0.49,
-// 32768: 0.97, 65536: 1.54 vs 1.46 one-threaded).  merkle_autotune_leaves
-// replaces them by measurement per (tree size, permutations per leaf).
-constexpr uint64_t kHexLeaves = 1 << 13, kDuoLeaves = 1 << 14;
+// pairs) or 1.  Static thresholds, measured on whole trees of 135-word leaves
+// (us, six / two / one threads per leaf): 4096 leaves 253 / 297 / -, 8192
+// 338 / 310 / -, 16384 586 / 421 / 453, 32768 - / 715 / 607.
+// merkle_autotune_leaves replaces them by measurement per (tree size,
+// permutations per leaf).  Poseidon2 has no two-thread form: six up to 8192
+// leaves (374 against 423 us one-threaded; 16384: 640 against 441).
+constexpr uint64_t kHexLeaves = 1 << 12, kDuoLeaves = 1 << 14, kHexLeaves2 = 1 << 13;
 constexpr uint64_t kLayoutTuneMax = 1 << 16;  // larger trees: one thread per hash, by a wide margin
 std::mutex g_layout_mu;
 std::map<uint64_t, uint8_t> g_layout;  // layout_key -> threads per hash
@@ -272,17 +335,16 @@ void merkle_run_t(const MerkleJob &j, cudaStream_t st) {
     if constexpr (H == kPoseidon || H == kPoseidon2) {
         // Latency-bound parts on several threads per hash: the leaves of
         // small trees (leaf_layout for Poseidon; Poseidon2 has the six-thread
-        // form only, up to kHexLeaves), levels of fewer than kHexNodes nodes,
+        // form only, up to kHexLeaves2), levels of fewer than kHexNodes nodes,
         // and the top (<= 32 nodes per subtree, so that one SM per subtree
-        // stays latency- rather than issue-bound) in one launch.  Measured
-        // per Poseidon level: 16384 nodes 46 us six-threaded vs 40 us
-        // one-threaded (issue bound: six threads do twice the instructions of
-        // one); 4096 nodes 20 us vs 40 us.
+        // stays latency- rather than issue-bound) in one launch.  Whole trees
+        // of 65536 8-word leaves with the line at 2^12, 2^13, 2^14 and 2^15
+        // nodes: Poseidon 225, 215, 211 and 221 us, Poseidon2 243, 235, 231 and 242.
         constexpr uint64_t kHexNodes = 1 << 14;
         if constexpr (H == kPoseidon) {
             launch_poseidon_leaves(j.leaves, j.n_leaves, w, j.digests, map, leaf_layout(j.n_leaves, w), st);
         } else {
-            if (j.n_leaves <= kHexLeaves)
+            if (j.n_leaves <= kHexLeaves2)
                 merkle_leaves_hex<H><<<hex_blocks(j.n_leaves), kHexThreads, 0, st>>>(j.leaves, j.n_leaves, w,
                                                                                      j.digests, map);
             else
@@ -310,22 +372,51 @@ void merkle_run_t(const MerkleJob &j, cudaStream_t st) {
                      w_top);
         return;
     }
-    merkle_leaves<H><<<blocks_for(j.n_leaves, kLeafThreads), kLeafThreads, 0, st>>>(j.leaves, j.n_leaves, w, j.digests,
-                                                                                     map);
-    ZK_CHECK_LAUNCH();
-    // Wide levels: one launch each, one node per thread.  The narrow top
-    // (fewer than kNarrow nodes in all, at most 256 per subtree) goes to
-    // merkle_top in one launch.
-    constexpr uint64_t kNarrow = 1 << 14;
-    uint32_t lg_top = 0;
-    while (lg_top + 1 < map.lg_ls && lg_top < 8 && (j.n_caps << (lg_top + 1)) < kNarrow) lg_top++;
-    for (uint32_t lg_w = map.lg_ls - 1; lg_w > lg_top; lg_w--)
-        launch_after(merkle_level<H, 4>, blocks_for(j.n_caps << lg_w, kLeafThreads), kLeafThreads, 0, st, j.digests,
-                     lg_w, j.n_caps, ds);
-    require(j.n_caps < (1ull << 31), "too many subtrees");
-    const uint32_t w_top = 1u << lg_top;
-    launch_after(merkle_top<H>, (unsigned)j.n_caps, std::max<uint32_t>(32, w_top), 0, st, j.digests, j.cap, ds,
-                 w_top);
+    if constexpr (H == kPoseidonBN128) {
+        // Five threads per hash up to 4096 hashes: there the GPU has a warp or
+        // two per scheduler either way, and a warp's time is its multiplies
+        // (level of 4096 nodes 0.22 ms against 0.49 one-threaded; 8192 leaves of
+        // 135 words 8.7 ms either way; 16384 leaves 14.5 against 8.9).
+        constexpr uint64_t kBnHashes = 1 << 12;
+        if (j.n_leaves <= kBnHashes)
+            merkle_leaves_bn<<<bn_blocks(j.n_leaves), kBnThreads, 0, st>>>(j.leaves, j.n_leaves, w, j.digests, map);
+        else
+            merkle_leaves<H><<<blocks_for(j.n_leaves, kLeafThreads), kLeafThreads, 0, st>>>(j.leaves, j.n_leaves, w,
+                                                                                             j.digests, map);
+        ZK_CHECK_LAUNCH();
+        uint32_t lg_top = 0;
+        while (lg_top + 1 < map.lg_ls && lg_top < 4 && (j.n_caps << (lg_top + 1)) < kBnHashes) lg_top++;
+        for (uint32_t lg_w = map.lg_ls - 1; lg_w > lg_top; lg_w--) {
+            const uint64_t nodes = j.n_caps << lg_w;
+            if (nodes > kBnHashes)
+                launch_after(merkle_level<H, 4>, blocks_for(nodes, kLeafThreads), kLeafThreads, 0, st, j.digests,
+                             lg_w, j.n_caps, ds);
+            else
+                launch_after(merkle_level_bn, bn_blocks(nodes), kBnThreads, 0, st, j.digests, lg_w, j.n_caps, ds);
+        }
+        require(j.n_caps < (1ull << 31), "too many subtrees");
+        const uint32_t w_top = 1u << lg_top;
+        launch_after(merkle_top_bn, (unsigned)j.n_caps, 32 * ((w_top + 5) / 6), 0, st, j.digests, j.cap, ds, w_top);
+        return;
+    }
+    if constexpr (H == kKeccak || H == kMonolith) {
+        merkle_leaves<H><<<blocks_for(j.n_leaves, kLeafThreads), kLeafThreads, 0, st>>>(j.leaves, j.n_leaves, w, j.digests,
+                                                                                         map);
+        ZK_CHECK_LAUNCH();
+        // Wide levels: one launch each, one node per thread.  The narrow top
+        // (fewer than kNarrow nodes in all, at most 256 per subtree) goes to
+        // merkle_top in one launch.
+        constexpr uint64_t kNarrow = 1 << 14;
+        uint32_t lg_top = 0;
+        while (lg_top + 1 < map.lg_ls && lg_top < 8 && (j.n_caps << (lg_top + 1)) < kNarrow) lg_top++;
+        for (uint32_t lg_w = map.lg_ls - 1; lg_w > lg_top; lg_w--)
+            launch_after(merkle_level<H, 4>, blocks_for(j.n_caps << lg_w, kLeafThreads), kLeafThreads, 0, st, j.digests,
+                         lg_w, j.n_caps, ds);
+        require(j.n_caps < (1ull << 31), "too many subtrees");
+        const uint32_t w_top = 1u << lg_top;
+        launch_after(merkle_top<H>, (unsigned)j.n_caps, std::max<uint32_t>(32, w_top), 0, st, j.digests, j.cap, ds,
+                     w_top);
+    }
 }
 
 }  // namespace
