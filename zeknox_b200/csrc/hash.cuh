@@ -450,35 +450,72 @@ __device__ __forceinline__ void poseidon2_permute(uint64_t s[12], const Poseidon
 }
 
 // --------------------------------------------------------------- Keccak
-__device__ __forceinline__ uint64_t rotl64(uint64_t x, int s) {
-    return s == 0 ? x : ((x << s) | (x >> (64 - s)));
+// Keccak-f on 32-bit halves with each three-input operation written as one
+// lop3 and each rotation as two funnel shifts.  Bound by the ALU pipe (97 %
+// busy): from 64-bit words the compiler made about 220 ALU instructions and 28
+// moves a round where 180 do.  Tree 2^18 x 135: 0.771 -> 0.645 ms.
+__device__ __forceinline__ uint32_t xor3(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0x96;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
 }
-
+__device__ __forceinline__ uint32_t chi3(uint32_t a, uint32_t b, uint32_t c) {  // a ^ (~b & c)
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xd2;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
+}
+template <int S>
+__device__ __forceinline__ void rotl_words(uint32_t &o0, uint32_t &o1, uint32_t l, uint32_t h) {
+    if constexpr (S == 0) o0 = l, o1 = h;
+    else if constexpr (S < 32) o0 = __funnelshift_l(h, l, S), o1 = __funnelshift_l(l, h, S);
+    else o0 = __funnelshift_l(l, h, S - 32), o1 = __funnelshift_l(h, l, S - 32);
+}
+template <int I>
+__device__ __forceinline__ void keccak_rho_pi(const uint32_t l[25], const uint32_t h[25], uint32_t bl[25], uint32_t bh[25]) {
+    if constexpr (I < 25) {
+        constexpr int rho[25] = {ZK_KECCAK_RHO_LIST};
+        constexpr int x = I % 5, y = I / 5, d = y + 5 * ((2 * x + 3 * y) % 5);
+        rotl_words<rho[I]>(bl[d], bh[d], l[I], h[I]);
+        keccak_rho_pi<I + 1>(l, h, bl, bh);
+    }
+}
 __device__ __forceinline__ void keccak_f1600(uint64_t a[25]) {
-    constexpr int rho[25] = {ZK_KECCAK_RHO_LIST};
+    uint32_t l[25], h[25];
+#pragma unroll
+    for (int i = 0; i < 25; i++) l[i] = (uint32_t)a[i], h[i] = (uint32_t)(a[i] >> 32);
 #pragma unroll 1
     for (int rnd = 0; rnd < 24; rnd++) {
-        uint64_t c[5], b[25];
-#pragma unroll
-        for (int x = 0; x < 5; x++) c[x] = a[x] ^ a[x + 5] ^ a[x + 10] ^ a[x + 15] ^ a[x + 20];
+        uint32_t cl[5], ch[5], bl[25], bh[25];
 #pragma unroll
         for (int x = 0; x < 5; x++) {
-            const uint64_t e = c[(x + 4) % 5], f = rotl64(c[(x + 1) % 5], 1);
+            cl[x] = xor3(xor3(l[x], l[x + 5], l[x + 10]), l[x + 15], l[x + 20]);
+            ch[x] = xor3(xor3(h[x], h[x + 5], h[x + 10]), h[x + 15], h[x + 20]);
+        }
 #pragma unroll
-            for (int y = 0; y < 25; y += 5) a[x + y] = a[x + y] ^ e ^ f;
+        for (int x = 0; x < 5; x++) {
+            uint32_t fl, fh;
+            rotl_words<1>(fl, fh, cl[(x + 1) % 5], ch[(x + 1) % 5]);
+#pragma unroll
+            for (int y = 0; y < 25; y += 5) {
+                l[x + y] = xor3(l[x + y], cl[(x + 4) % 5], fl);
+                h[x + y] = xor3(h[x + y], ch[(x + 4) % 5], fh);
+            }
         }
         // rho + pi: B[y, 2x + 3y] = rot(A[x, y], rho[x, y])
-#pragma unroll
-        for (int x = 0; x < 5; x++)
-#pragma unroll
-            for (int y = 0; y < 5; y++) b[y + 5 * ((2 * x + 3 * y) % 5)] = rotl64(a[x + 5 * y], rho[x + 5 * y]);
+        keccak_rho_pi<0>(l, h, bl, bh);
         // chi
 #pragma unroll
         for (int y = 0; y < 25; y += 5)
 #pragma unroll
-            for (int x = 0; x < 5; x++) a[x + y] = b[x + y] ^ (~b[(x + 1) % 5 + y] & b[(x + 2) % 5 + y]);
-        a[0] ^= c_keccak_rc[rnd];
+            for (int x = 0; x < 5; x++) {
+                l[x + y] = chi3(bl[x + y], bl[(x + 1) % 5 + y], bl[(x + 2) % 5 + y]);
+                h[x + y] = chi3(bh[x + y], bh[(x + 1) % 5 + y], bh[(x + 2) % 5 + y]);
+            }
+        l[0] ^= (uint32_t)c_keccak_rc[rnd];
+        h[0] ^= (uint32_t)(c_keccak_rc[rnd] >> 32);
     }
+#pragma unroll
+    for (int i = 0; i < 25; i++) a[i] = ((uint64_t)h[i] << 32) | l[i];
 }
 
 // --------------------------------------------------------------- Monolith
