@@ -187,6 +187,83 @@ def test_two_partial_rounds_at_once(seed):
         assert out == want
 
 
+@pytest.mark.parametrize("seed", range(3))
+def test_three_partial_rounds_at_once(seed):
+    """The triple's integer sums, as the one-thread kernel forms them, against three plain rounds; every sum below 2^53."""
+    rc, circ, diag = poseidon_constants()
+    conv = lambda a: [sum(a[i] * circ[(j - i) % 12] for i in range(12)) for j in range(12)]  # noqa: E731
+    row = {1: circ, 2: conv(circ), 3: conv(conv(circ))}
+    at = lambda n, j: row[n][j % 12]  # noqa: E731
+    kappa, d = 2755704, diag[0]
+    pm = lambda n, r, k: at(n, k - r) + at(n, k + 6 - r) - (kappa if n == 3 else 0)  # noqa: E731
+    qm = lambda n, r, k: at(n, k - r) - at(n, k + 6 - r)  # noqa: E731
+    offset = lambda n, r: (1 if r < 6 else -1) * 2**31 * sum(qm(n, r % 6, k) for k in range(6))  # noqa: E731
+    mds = lambda x: [(sum(circ[(k - r) % 12] * x[k] for k in range(12)) + (d * x[0] if r == 0 else 0)) % P for r in range(12)]  # noqa: E731
+    half = lambda v, h: v >> 32 if h else v & M32  # noqa: E731
+    rnd = random.Random(seed)
+
+    def exact(*v):
+        assert all(abs(x) < 2**53 for x in v)
+        return v[0]
+
+    def rows(n, u, w, t=0):
+        """4 C^n x + t by the 3x3 split; every partial sum bounded."""
+        up, um = [u[i] + u[i + 3] for i in range(3)], [u[i] - u[i + 3] for i in range(3)]
+        out = [0] * 12
+        for r in range(3):
+            ps = [(pm(n, r, k) + pm(n, r, k + 3)) * up[k] for k in range(3)]
+            pd = [(pm(n, r, k) - pm(n, r, k + 3)) * um[k] for k in range(3)]
+            exact(*[abs(t) + sum(map(abs, ps))], *[sum(map(abs, pd))])
+            sp, sm = t + sum(ps), sum(pd)
+            for rr, pa in ((r, sp + sm), (r + 3, sp - sm)):
+                q = [2 * qm(n, rr, k) * w[k] for k in range(6)]
+                qa = sum(q)
+                exact(pa, sum(map(abs, q)), pa + qa, pa - qa)
+                assert (pa + qa) % 4 == (pa - qa) % 4 == 0
+                out[rr], out[rr + 6] = (pa + qa) // 4, (pa - qa) // 4
+        return out
+
+    for q in range(7):
+        fill = rnd.choice([0, 2**64 - 1, None])  # all lanes at an end of their range, or mixed
+        x = [rnd.choice([rnd.getrandbits(64), 2**64 - 1, 0, M32, M32 << 32, P - 1]) if fill is None else fill for _ in range(12)]
+        if q % 2:
+            x = [2**64 - 1 if i in (0, 3, 6, 9) else 0 for i in range(12)]  # the signs of C^3 - kappa / 2
+        want = list(x)
+        for j in range(3):
+            want[0] = pow(want[0], 7, P)
+            want = [(a + b) % P for a, b in zip(mds(want), rc[12 * (5 + 3 * q + j):])]
+        c = rc[12 * (5 + 3 * q):][:12]
+        ctimes = lambda v: [sum(circ[(k - r) % 12] * v[k] for k in range(12)) % P for r in range(12)]  # noqa: E731
+        c2 = [(a + b) % P for a, b in zip(ctimes(c), rc[12 * (6 + 3 * q):])]
+        c3 = [(a + b) % P for a, b in zip(ctimes(c2), rc[12 * (7 + 3 * q):])]
+
+        s = [pow7(x[0])] + x[1:]
+        u = [[half(s[i], h) + half(s[i + 6], h) for i in range(6)] for h in (0, 1)]
+        w = [[half(s[i], h) - half(s[i + 6], h) + 2**32 for i in range(6)] for h in (0, 1)]
+        ky, kz = kpair(c[0], offset(1, 0), 2**40), kpair(c2[0], offset(2, 0), 2**45)
+        y = [exact(rows(1, u[h], w[h])[0] + d * half(s[0], h) + ky[h]) for h in (0, 1)]
+        assert min(y) >= 0
+        yr = pr_reduce_split_add(*y)
+        yp = pow7(yr)
+        total = pr_reduce_split_add(sum(u[0]), sum(u[1]))
+        t = pr_reduce_split_add(*[exact(kappa // 2 * half(total, h)) for h in (0, 1)])
+        g0 = [d * half(s[0], h) + half(yp, h) - half(yr, h) for h in (0, 1)]
+        z = [exact(rows(2, u[h], w[h])[0] + kz[h] + d * half(yp, h) + circ[0] * g0[h]) for h in (0, 1)]
+        assert min(z) >= 0
+        zr = pr_reduce_split_add(*z)
+        zq = pow7(zr)
+        out = [[], []]
+        for h in (0, 1):
+            g1 = d * half(yp, h) + half(zq, h) - half(zr, h)
+            for r, v in enumerate(rows(3, u[h], w[h], 4 * half(t, h))):
+                v = exact(v + kpair(c3[r], offset(3, r), 2**49)[h])
+                v = exact(v + at(2, -r) * g0[h], at(2, -r) * g0[h])
+                v = exact(v + at(1, -r) * g1 + (d * half(zq, h) if r == 0 else 0))
+                assert v >= 0
+                out[h].append(v)
+        assert [pr_reduce_split_add(a, b) % P for a, b in zip(*out)] == want
+
+
 BN_R = 0x30644E72E131A029B85045B68181585D2833E84879B9709143E1F593F0000001
 MASK = 2**29 - 1
 

@@ -260,10 +260,13 @@ __device__ __forceinline__ uint64_t mont_sqr(uint64_t a) {  // a^2 2^-64
 // With R = 2^64: x^2 R^-1, x^3 R^-2, x^4 R^-3 and their product x^7 R^-6; 2 has
 // order 192 mod p, so R^3 = 1 and the result is x^7 itself: no conversion in
 // or out.  Per application 62 instructions; with the folding reduction 86.
+// kMulSqr: the squares as plain products, three ALU instructions fewer for one
+// multiply more each.
+template <bool kMulSqr = false>
 __device__ __forceinline__ uint64_t pr_pow7(uint64_t x) {
-    const uint64_t x2 = mont_sqr(x);
+    const uint64_t x2 = kMulSqr ? mont_mul(x, x) : mont_sqr(x);
     const uint64_t x3 = mont_mul(x, x2);
-    const uint64_t x4 = mont_sqr(x2);
+    const uint64_t x4 = kMulSqr ? mont_mul(x2, x2) : mont_sqr(x2);
     return mont_mul(x3, x4);
 }
 

@@ -71,19 +71,50 @@ struct RcTable {
 template <class H>
 struct Circ {  // H::c(j), j in 0..11: the first row; H::d0(): the diagonal term
     __host__ __device__ static constexpr int at(int j) { return H::c(((j % 12) + 12) % 12); }
-    __host__ __device__ static constexpr int at2(int j) {  // first row of C^2
-        int v = 0;
-        for (int i = 0; i < 12; i++) v += at(i) * at(j - i);
-        return v;
+    struct Row {
+        int v[12];
+    };
+    static constexpr Row power_row(int n) {  // first row of C^n
+        Row p{};
+        for (int j = 0; j < 12; j++) p.v[j] = H::c(j);
+        for (; n > 1; n--) {
+            Row t{};
+            for (int i = 0; i < 12; i++)
+                for (int j = 0; j < 12; j++) t.v[(i + j) % 12] += p.v[i] * H::c(j);
+            p = t;
+        }
+        return p;
     }
-    // entries of A + B and A - B, of C (N = 1) or C^2 (N = 2)
+    template <int N>
+    __host__ __device__ static constexpr int atn(int j) {
+        constexpr Row p = power_row(N);
+        return p.v[((j % 12) + 12) % 12];
+    }
+    // entries of A + B (less kappa, a multiple of the all-ones matrix) and A - B, of C^N
     template <int N>
     __host__ __device__ static constexpr int p(int r, int k) {
-        return N == 1 ? at(k - r) + at(k + 6 - r) : at2(k - r) + at2(k + 6 - r);
+        return atn<N>(k - r) + atn<N>(k + 6 - r) - kappa<N>();
     }
     template <int N>
     __host__ __device__ static constexpr int q(int r, int k) {
-        return N == 1 ? at(k - r) - at(k + 6 - r) : at2(k - r) - at2(k + 6 - r);
+        return atn<N>(k - r) - atn<N>(k + 6 - r);
+    }
+    // 2^18 times 2^33 is what fits: the entries of C^3 only do once most of their
+    // common value is taken out (any even number will do; near the median, least is left)
+    template <int N>
+    __host__ __device__ static constexpr int kappa() {
+        if constexpr (N == 3) return H::kappa3();
+        else return 0;
+    }
+    // A + B is a 6x6 circulant [[E, F], [F, E]]: the same split once more, with
+    // E + F on u_i + u_(i+3) and E - F on u_i - u_(i+3)
+    template <int N>
+    __host__ __device__ static constexpr double ps(int r, int k) {
+        return p<N>(r, k) + p<N>(r, k + 3);
+    }
+    template <int N>
+    __host__ __device__ static constexpr double pd(int r, int k) {
+        return p<N>(r, k) - p<N>(r, k + 3);
     }
     // what the offset of w adds to output row r of either half-vector
     template <int N>
@@ -122,36 +153,95 @@ __device__ __forceinline__ double diff_dbl(uint32_t a, uint32_t b) {
 }
 __device__ __forceinline__ uint32_t half_of(uint64_t x, int h) { return h ? (uint32_t)(x >> 32) : (uint32_t)x; }
 
-// Half h of the lanes s through the layer: o[r] = k[r] + (C x)[r] + [r = 0] d x[0].
-template <class H>
-__device__ __forceinline__ void circ_half(const uint64_t s[12], int h, double o[12], const uint64_t *k) {
-    using C = Circ<H>;
+// Half h of the lanes as the split takes it: w, and u or (H::split3) its sums
+// and differences u_i + u_(i+3), u_i - u_(i+3).
+struct CircIn {
     double u[6], w[6];
+};
+template <class H>
+__device__ __forceinline__ CircIn circ_in(const uint64_t s[12], int h) {
+    CircIn x;
 #pragma unroll
-    for (int i = 0; i < 6; i++) {
-        u[i] = sum_dbl(half_of(s[i], h), half_of(s[i + 6], h));
-        w[i] = diff_dbl(half_of(s[i], h), half_of(s[i + 6], h));
+    for (int i = 2; i >= 0; i--) {
+        const double a = sum_dbl(half_of(s[i], h), half_of(s[i + 6], h));
+        const double b = sum_dbl(half_of(s[i + 3], h), half_of(s[i + 9], h));
+        x.u[i] = H::split3() ? a + b : a;
+        x.u[i + 3] = H::split3() ? a - b : b;
+        x.w[i] = diff_dbl(half_of(s[i], h), half_of(s[i + 6], h));
+        x.w[i + 3] = diff_dbl(half_of(s[i + 3], h), half_of(s[i + 9], h));
+    }
+    return x;
+}
+// f(r, value) for the 12 rows of C^N x + k (+ t / 4 on every row); lane 0, the
+// last to leave an S-box, comes last in every sum.
+template <class H, int N, class F>
+__device__ __forceinline__ void circ_rows(const CircIn &x, const uint64_t *k, double t, F &&f) {
+    using C = Circ<H>;
+    if constexpr (!H::split3()) {
+#pragma unroll
+        for (int r = 0; r < 6; r++) {
+            double pa = (double)C::template p<N>(r, 0) * x.u[0], qa = (double)C::template q<N>(r, 0) * x.w[0];
+#pragma unroll
+            for (int c = 1; c < 6; c++) {
+                pa = fma((double)C::template p<N>(r, c), x.u[c], pa);
+                qa = fma((double)C::template q<N>(r, c), x.w[c], qa);
+            }
+            f(r, fma(0.5, pa + qa, int_dbl(k[r])));
+            f(r + 6, fma(0.5, pa - qa, int_dbl(k[r + 6])));
+        }
+        return;
     }
 #pragma unroll
-    for (int r = 0; r < 6; r++) {
-        double pa = (double)C::template p<1>(r, 0) * u[0], qa = (double)C::template q<1>(r, 0) * w[0];
+    for (int r = 0; r < 3; r++) {
+        double sp = N == 3 ? fma(C::template ps<N>(r, 2), x.u[2], t) : C::template ps<N>(r, 2) * x.u[2];
+        double sm = C::template pd<N>(r, 2) * x.u[5];
 #pragma unroll
-        for (int c = 1; c < 6; c++) {
-            pa = fma((double)C::template p<1>(r, c), u[c], pa);
-            qa = fma((double)C::template q<1>(r, c), w[c], qa);
+        for (int c = 1; c >= 0; c--) {
+            sp = fma(C::template ps<N>(r, c), x.u[c], sp);
+            sm = fma(C::template pd<N>(r, c), x.u[c + 3], sm);
         }
-        o[r] = fma(0.5, pa + qa, int_dbl(k[r]));
-        if (H::d0() != 0 && r == 0) o[0] = fma((double)H::d0(), word_dbl(half_of(s[0], h)), o[0]);
-        o[r + 6] = fma(0.5, pa - qa, int_dbl(k[r + 6]));
+#pragma unroll
+        for (int e = 0; e < 2; e++) {  // rows r and r + 3 of A + B: 2 (A + B) u = sp +- sm
+            const int rr = r + 3 * e;
+            const double pa = e ? sp - sm : sp + sm;
+            double qa = (double)(2 * C::template q<N>(rr, 5)) * x.w[5];
+#pragma unroll
+            for (int c = 4; c >= 0; c--) qa = fma((double)(2 * C::template q<N>(rr, c)), x.w[c], qa);
+            f(rr, fma(0.25, pa + qa, int_dbl(k[rr])));
+            f(rr + 6, fma(0.25, pa - qa, int_dbl(k[rr + 6])));
+        }
     }
 }
+// 4 times row 0 of C^N x
+template <class H, int N>
+__device__ __forceinline__ double circ_row0(const CircIn &x) {
+    using C = Circ<H>;
+    double a = C::template ps<N>(0, 2) * x.u[2], b = C::template pd<N>(0, 2) * x.u[5];
+    double c = (double)(2 * C::template q<N>(0, 5)) * x.w[5];
+#pragma unroll
+    for (int i = 4; i > 0; i--) c = fma((double)(2 * C::template q<N>(0, i)), x.w[i], c);
+    a = fma(C::template ps<N>(0, 1), x.u[1], a);
+    b = fma(C::template pd<N>(0, 1), x.u[4], b);
+    a = fma(C::template ps<N>(0, 0), x.u[0], a);
+    b = fma(C::template pd<N>(0, 0), x.u[3], b);
+    c = fma((double)(2 * C::template q<N>(0, 0)), x.w[0], c);
+    return (a + b) + c;
+}
+
 template <class H>
 __device__ __forceinline__ void circ_layer(uint64_t s[12], const uint64_t (*k)[12]) {
-    double lo[12], hi[12];
-    circ_half<H>(s, 0, lo, k[0]);
-    circ_half<H>(s, 1, hi, k[1]);
-#pragma unroll
-    for (int r = 0; r < 12; r++) s[r] = pr_reduce_split(dbl_int(lo[r]), dbl_int(hi[r]));
+    double lo[12];
+    {
+        const CircIn x = circ_in<H>(s, 0);
+        circ_rows<H, 1>(x, k[0], 0.0, [&](int r, double v) { lo[r] = v; });
+        if (H::d0() != 0) lo[0] = fma((double)H::d0(), word_dbl((uint32_t)s[0]), lo[0]);
+    }
+    const uint64_t x0 = s[0];
+    const CircIn x = circ_in<H>(s, 1);
+    circ_rows<H, 1>(x, k[1], 0.0, [&](int r, double v) {
+        if (H::d0() != 0 && r == 0) v = fma((double)H::d0(), word_dbl((uint32_t)(x0 >> 32)), v);
+        s[r] = pr_reduce_split(dbl_int(lo[r]), dbl_int(v));
+    });
 }
 
 // ------------------------------------------------------------ Poseidon
@@ -165,6 +255,8 @@ struct PoseidonMds {
         constexpr uint32_t diag[12] = {ZK_POSEIDON_MDS_DIAG_LIST};
         return (int)diag[0];
     }
+    __host__ __device__ static constexpr int kappa3() { return 2755704; }
+    __host__ __device__ static constexpr bool split3() { return true; }
 };
 using PoseidonCirc = Circ<PoseidonMds>;
 constexpr bool diag_only_lane0() {
@@ -179,47 +271,89 @@ static_assert(diag_only_lane0(), "the MDS layer below assumes diag(d, 0, ..., 0)
 // 26-29, lane 0 otherwise) and the MDS layer M = C + d e0 e0^T.  Constants of
 // round r + 1 are added inside round r's layer.
 //
-// The 22 partial rounds run two at a time.  With x the state, x0' = S(x0),
-// c, c' the next two rounds' constants, y0 = (M x')_0 + c_0 and y0' = S(y0):
+// The 22 partial rounds run several at a time, so that one layer's work covers
+// them.  Two rounds, with x the state, x0' = S(x0), c, c' the next rounds'
+// constants, y0 = (M x')_0 + c_0 and y0' = S(y0):
 //   M (M x' + c + (y0' - y0) e0) + c'
 //     = C^2 x' + g C e0 + d y0' e0 + (C c + c'),    g = d x0' + y0' - y0,
-// one layer's work for two rounds plus one row for y0 and one column for g.
-// C^2 has entries below 2^13 and row sums of 2^16, so every sum stays below
-// 2^50.  g and y0 stay split in (unreduced) halves.
-struct PoseidonTab {
-    uint64_t full[8][2][12];   // layers of rounds 0-3 and 26-29 (no constants after 29)
+// plus one row for y0 and one column for g.  Three rounds go on from there with
+// z0 = (C^2 x')_0 + g C_00 + d y0' + .., z0' = S(z0) and g' = d y0' + z0' - z0:
+//     = C^3 x' + g C^2 e0 + g' C e0 + d z0' e0 + (C^2 c + C c' + c'').
+// C^2 has row sums of 2^16; those of C^3 are 2^24, and with halves of 2^33 only
+// its entries less their common part kappa / 2 stay exact (sums below 2^53):
+// kappa / 2 times the sum of the lanes is formed mod p and added to every row.
+// One thread per hash takes three rounds at a time (rounds 4-24, and 25 alone);
+// the forms on several threads take two, whose dependent chain is the same
+// length per round but whose tables fit their shared memory copies better.
+struct PoseidonTab {          // one thread per hash
+    uint64_t full[9][2][12];  // layers of rounds 0-3 and 25-29 (no constants after 29)
+    uint64_t trip[7][2][12];  // layers of rounds (4, 5, 6) .. (22, 23, 24)
+    uint64_t mid[7][2][2];    // y0 and z0 of each
+    uint64_t rc0[12];         // round 0, added before the first S-box
+};
+struct PoseidonGroupTab {      // several threads per hash
+    uint64_t full[8][2][12];   // layers of rounds 0-3 and 26-29
     uint64_t pair[11][2][12];  // layers of round pairs (4, 5) .. (24, 25)
     uint64_t mid[11][2];       // y0 of each pair
-    uint64_t rc0[12];          // round 0, added before the first S-box
+    uint64_t rc0[12];
     // the six-thread form's rows t of A + B and A - B (for C and C^2), and C e0 at rows t and t + 6
     double rows[6][26];
 };
 constexpr uint64_t kFullBias = 1ull << 40;  // above the w offset of C: 113 * 2^31
 constexpr uint64_t kPairBias = 1ull << 48;  // above 41 * 2^42 of -g and the w offset of C^2
+constexpr uint64_t kTripBias = 1ull << 49;  // above 2^33 times the negative entries of (C^3 - kappa / 2)
+struct Vec12 {
+    uint64_t v[12];
+};
+constexpr Vec12 circ_times(const Vec12 &x) {  // C x mod p
+    Vec12 y{};
+    for (int r = 0; r < 12; r++)
+        for (int j = 0; j < 12; j++)
+            y.v[r] = cx_add_mod(y.v[r], cx_mul_mod(x.v[j], (uint64_t)PoseidonCirc::at(j - r)));
+    return y;
+}
+constexpr Vec12 plus_rc(const Vec12 &x, const RcTable &rc, int rnd) {  // x + round rnd's constants
+    Vec12 y{};
+    for (int i = 0; i < 12; i++) y.v[i] = cx_add_mod(x.v[i], rnd < 30 ? cx_canon(rc.v[12 * rnd + i]) : 0);
+    return y;
+}
+template <int N>
+constexpr void put_layer(uint64_t (&to)[2][12], const Vec12 &k, uint64_t bias) {
+    for (int r = 0; r < 12; r++) {
+        const KPair p = make_kpair(k.v[r], PoseidonCirc::offset<N>(r), bias);
+        to[0][r] = p.lo;
+        to[1][r] = p.hi;
+    }
+}
 constexpr PoseidonTab make_poseidon_tab(RcTable rc) {
     PoseidonTab t{};
     for (int i = 0; i < 12; i++) t.rc0[i] = cx_canon(rc.v[i]);
-    for (int f = 0; f < 8; f++) {
-        const int rnd = f < 4 ? f : 22 + f;
-        for (int r = 0; r < 12; r++) {
-            const KPair k = make_kpair(rnd < 29 ? rc.v[12 * (rnd + 1) + r] : 0, PoseidonCirc::offset<1>(r), kFullBias);
-            t.full[f][0][r] = k.lo;
-            t.full[f][1][r] = k.hi;
-        }
+    for (int f = 0; f < 9; f++) put_layer<1>(t.full[f], plus_rc(Vec12{}, rc, (f < 4 ? f : 21 + f) + 1), kFullBias);
+    for (int q = 0; q < 7; q++) {
+        const int rnd = 4 + 3 * q;
+        const Vec12 c = plus_rc(Vec12{}, rc, rnd + 1), c2 = plus_rc(circ_times(c), rc, rnd + 2),
+                    c3 = plus_rc(circ_times(c2), rc, rnd + 3);
+        const KPair y = make_kpair(c.v[0], PoseidonCirc::offset<1>(0), kFullBias);
+        const KPair z = make_kpair(c2.v[0], PoseidonCirc::offset<2>(0), kFullBias << 5);
+        t.mid[q][0][0] = y.lo;
+        t.mid[q][0][1] = y.hi;
+        t.mid[q][1][0] = z.lo;
+        t.mid[q][1][1] = z.hi;
+        put_layer<3>(t.trip[q], c3, kTripBias);
     }
+    return t;
+}
+constexpr PoseidonGroupTab make_poseidon_group_tab(RcTable rc) {
+    PoseidonGroupTab t{};
+    for (int i = 0; i < 12; i++) t.rc0[i] = cx_canon(rc.v[i]);
+    for (int f = 0; f < 8; f++) put_layer<1>(t.full[f], plus_rc(Vec12{}, rc, (f < 4 ? f : 22 + f) + 1), kFullBias);
     for (int q = 0; q < 11; q++) {
-        const uint64_t *c = &rc.v[12 * (5 + 2 * q)], *c2 = &rc.v[12 * (6 + 2 * q)];
-        const KPair m = make_kpair(c[0], PoseidonCirc::offset<1>(0), kFullBias);
-        t.mid[q][0] = m.lo;
-        t.mid[q][1] = m.hi;
-        for (int r = 0; r < 12; r++) {
-            uint64_t v = cx_canon(c2[r]);
-            for (int j = 0; j < 12; j++)
-                v = cx_add_mod(v, cx_mul_mod(cx_canon(c[j]), (uint64_t)PoseidonCirc::at(j - r)));
-            const KPair k = make_kpair(v, PoseidonCirc::offset<2>(r), kPairBias);
-            t.pair[q][0][r] = k.lo;
-            t.pair[q][1][r] = k.hi;
-        }
+        const int rnd = 4 + 2 * q;
+        const Vec12 c = plus_rc(Vec12{}, rc, rnd + 1);
+        const KPair y = make_kpair(c.v[0], PoseidonCirc::offset<1>(0), kFullBias);
+        t.mid[q][0] = y.lo;
+        t.mid[q][1] = y.hi;
+        put_layer<2>(t.pair[q], plus_rc(circ_times(c), rc, rnd + 2), kPairBias);
     }
     for (int r = 0; r < 6; r++) {
         for (int k = 0; k < 6; k++) {
@@ -253,53 +387,48 @@ constexpr Poseidon2Tab make_poseidon2_tab(RcTable rc) {
 }
 __constant__ PoseidonTab c_poseidon = make_poseidon_tab(RcTable{{ZK_POSEIDON_RC_LIST}});
 __constant__ Poseidon2Tab c_poseidon2 = make_poseidon2_tab(RcTable{{ZK_POSEIDON2_RC_LIST}});
-__device__ PoseidonTab g_poseidon = make_poseidon_tab(RcTable{{ZK_POSEIDON_RC_LIST}});
+__device__ PoseidonGroupTab g_poseidon = make_poseidon_group_tab(RcTable{{ZK_POSEIDON_RC_LIST}});
 __device__ Poseidon2Tab g_poseidon2 = make_poseidon2_tab(RcTable{{ZK_POSEIDON2_RC_LIST}});
 __constant__ uint64_t c_keccak_rc[24] = {ZK_KECCAK_RC_LIST};
 __constant__ KeccakTab c_keccak_tab;
 
-// Two partial rounds (the pair q), see above.
-__device__ __forceinline__ void poseidon_pair(uint64_t s[12], int q, const PoseidonTab &tab) {
+// Three partial rounds (the triple q), see above.
+__device__ __forceinline__ void poseidon_triple(uint64_t s[12], int q, const PoseidonTab &tab) {
     using C = PoseidonCirc;
-    constexpr double d0 = (double)PoseidonMds::d0();
-    double u[2][6], w[2][6], y0[2], lo[12];
+    constexpr double d0 = (double)PoseidonMds::d0(), c00 = (double)C::at(0);
     s[0] = pr_pow7(s[0]);
+    const uint64_t x0 = s[0];
+    CircIn x[2];
+    double y[2], z[2], tau[2], g0[2], g1[2], zp[2], lo[12];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-        double pa = 0, qa = 0;
-#pragma unroll
-        for (int i = 5; i >= 0; i--) {  // lane 0, which has just left the S-box, last
-            u[h][i] = sum_dbl(half_of(s[i], h), half_of(s[i + 6], h));
-            w[h][i] = diff_dbl(half_of(s[i], h), half_of(s[i + 6], h));
-            pa = fma((double)C::p<1>(0, i), u[h][i], pa);
-            qa = fma((double)C::q<1>(0, i), w[h][i], qa);
-        }
-        y0[h] = fma(0.5, pa + qa, fma(d0, word_dbl(half_of(s[0], h)), int_dbl(tab.mid[q][h])));
+        x[h] = circ_in<PoseidonMds>(s, h);
+        y[h] = fma(0.25, circ_row0<PoseidonMds, 1>(x[h]), fma(d0, word_dbl(half_of(x0, h)), int_dbl(tab.mid[q][0][h])));
+        z[h] = fma(0.25, circ_row0<PoseidonMds, 2>(x[h]), int_dbl(tab.mid[q][1][h]));
+        tau[h] = x[h].u[2] + x[h].u[1] + x[h].u[0];
     }
-    const uint64_t x0 = s[0], y = pr_pow7(pr_reduce_split(dbl_int(y0[0]), dbl_int(y0[1])));
+    const uint64_t yr = pr_reduce_split(dbl_int(y[0]), dbl_int(y[1])), yp = pr_pow7(yr);
+    // kappa / 2 times the sum of the lanes, mod p
+    const uint64_t sum = pr_reduce_split(dbl_int(tau[0]), dbl_int(tau[1]));
+    constexpr double k2 = (double)(C::kappa<3>() / 2);
+    const uint64_t t = pr_reduce_split(dbl_int(k2 * word_dbl((uint32_t)sum)), dbl_int(k2 * word_dbl((uint32_t)(sum >> 32))));
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-        const double yp = word_dbl(half_of(y, h));
-        const double g = fma(d0, word_dbl(half_of(x0, h)), yp - y0[h]);
+        g0[h] = fma(d0, word_dbl(half_of(x0, h)), word_dbl(half_of(yp, h)) - word_dbl(half_of(yr, h)));
+        z[h] = fma(c00, g0[h], fma(d0, word_dbl(half_of(yp, h)), z[h]));
+    }
+    const uint64_t zr = pr_reduce_split(dbl_int(z[0]), dbl_int(z[1])), zq = pr_pow7(zr);
 #pragma unroll
-        for (int r = 0; r < 6; r++) {
-            double pa = (double)C::p<2>(r, 5) * u[h][5], qa = (double)C::q<2>(r, 5) * w[h][5];
-#pragma unroll
-            for (int c = 4; c >= 0; c--) {
-                pa = fma((double)C::p<2>(r, c), u[h][c], pa);
-                qa = fma((double)C::q<2>(r, c), w[h][c], qa);
-            }
-            double o0 = fma((double)C::at(-r), g, fma(0.5, pa + qa, int_dbl(tab.pair[q][h][r])));
-            const double o6 = fma((double)C::at(-r - 6), g, fma(0.5, pa - qa, int_dbl(tab.pair[q][h][r + 6])));
-            if (r == 0) o0 = fma(d0, yp, o0);
-            if (h == 0) {
-                lo[r] = o0;
-                lo[r + 6] = o6;
-            } else {
-                s[r] = pr_reduce_split(dbl_int(lo[r]), dbl_int(o0));
-                s[r + 6] = pr_reduce_split(dbl_int(lo[r + 6]), dbl_int(o6));
-            }
-        }
+    for (int h = 0; h < 2; h++) {
+        zp[h] = word_dbl(half_of(zq, h));
+        g1[h] = fma(d0, word_dbl(half_of(yp, h)), zp[h] - word_dbl(half_of(zr, h)));
+        circ_rows<PoseidonMds, 3>(x[h], tab.trip[q][h], 4.0 * word_dbl(half_of(t, h)), [&](int r, double v) {
+            v = fma((double)C::atn<2>(-r), g0[h], v);
+            v = fma((double)C::at(-r), g1[h], v);
+            if (r == 0) v = fma(d0, zp[h], v);
+            if (h == 0) lo[r] = v;
+            else s[r] = pr_reduce_split(dbl_int(lo[r]), dbl_int(v));
+        });
     }
 }
 
@@ -336,13 +465,14 @@ __device__ __forceinline__ void poseidon_permute(uint64_t s[12], const PoseidonT
 #pragma unroll 1
     for (int half = 0; half < 2; half++) {
 #pragma unroll 1
-        for (int f = 0; f < 4; f++) {
-            pow7_all<W>(s);
+        for (int f = 0; f < 4 + half; f++) {
+            if (half && f == 0) s[0] = pr_pow7(s[0]);  // round 25
+            else pow7_all<W>(s);
             circ_layer<PoseidonMds>(s, tab.full[4 * half + f]);
         }
         if (half) break;
 #pragma unroll 1
-        for (int q = 0; q < 11; q++) poseidon_pair(s, q, tab);
+        for (int q = 0; q < 7; q++) poseidon_triple(s, q, tab);
     }
 }
 
@@ -537,6 +667,8 @@ struct MonolithMds {
         return (int)row[j];
     }
     __host__ __device__ static constexpr int d0() { return 0; }
+    // its bytewise Bars keep the integer pipes busiest: the further split measured 1 % slower
+    __host__ __device__ static constexpr bool split3() { return false; }
 };
 
 // Accumulator starting values of the 7 concrete layers.
@@ -931,9 +1063,12 @@ __device__ __forceinline__ const typename TabOf<H>::type &const_tab() {
     else return c_keccak_tab;
 }
 
-// The __device__ twin of a hasher's tables (source of shared-memory copies).
+// The tables of the forms on several threads (and of one block per subtree),
+// copied to shared memory from their __device__ twin.
 template <int H>
-__device__ __forceinline__ const typename TabOf<H>::type *global_tab() {
+using GroupTabOf = typename std::conditional<H == kPoseidon, PoseidonGroupTab, typename TabOf<H>::type>::type;
+template <int H>
+__device__ __forceinline__ const GroupTabOf<H> *global_tab() {
     if constexpr (H == kPoseidon) return &g_poseidon;
     else if constexpr (H == kPoseidon2) return &g_poseidon2;
     else if constexpr (H == kMonolith) return &g_monolith;
@@ -992,7 +1127,8 @@ __device__ __forceinline__ void hash_two(const uint64_t *l, const uint64_t *r, u
 // partner's input halves, and six 64-bit shuffles hand each thread the other
 // half of its own lanes' outputs.  In a pair of partial rounds lane 0's first
 // S-box runs on thread 0 and its second one, after an exchange of the halves
-// of y0, on both threads.
+// of y0, on both threads.  The squares are plain products here (8192 x 135 tree
+// 310 -> 305 us; the six-thread form loses by that, 2048 x 135: 185 -> 230).
 __device__ __forceinline__ uint32_t shfl_xor32(uint32_t v) { return (uint32_t)__shfl_xor_sync(0xffffffffu, (int)v, 1); }
 __device__ __forceinline__ double shfl_xor_d(double v) { return __shfl_xor_sync(0xffffffffu, v, 1); }
 
@@ -1036,7 +1172,7 @@ __device__ __forceinline__ void duo_rows(const double u[6], const double w[6], d
 
 // s: lanes 6h .. 6h + 5 (partially reduced, in and out).  Every lane of the
 // warp must call this (shuffles over the full warp).
-__device__ __forceinline__ void poseidon_permute_duo(uint64_t s[6], uint32_t h, const PoseidonTab &tab) {
+__device__ __forceinline__ void poseidon_permute_duo(uint64_t s[6], uint32_t h, const PoseidonGroupTab &tab) {
     using C = PoseidonCirc;
     constexpr double d0 = (double)PoseidonMds::d0();
 #pragma unroll
@@ -1046,7 +1182,7 @@ __device__ __forceinline__ void poseidon_permute_duo(uint64_t s[6], uint32_t h, 
 #pragma unroll 1
         for (int f = 0; f < 4; f++) {
 #pragma unroll
-            for (int i = 0; i < 6; i++) s[i] = pr_pow7(s[i]);
+            for (int i = 0; i < 6; i++) s[i] = pr_pow7<true>(s[i]);
             double u[6], w[6], o[12];
             duo_inputs(s, h, u, w);
             duo_rows<1>(u, w, o, tab.full[4 * half + f][h]);
@@ -1057,7 +1193,7 @@ __device__ __forceinline__ void poseidon_permute_duo(uint64_t s[6], uint32_t h, 
         if (half) break;
 #pragma unroll 1
         for (int q = 0; q < 11; q++) {
-            if (h == 0) s[0] = pr_pow7(s[0]);
+            if (h == 0) s[0] = pr_pow7<true>(s[0]);
             double u[6], w[6], o[12];
             duo_inputs(s, h, u, w);
             const double x0 = 0.5 * (u[0] + (w[0] - int_dbl(1ull << 32)));
@@ -1069,7 +1205,7 @@ __device__ __forceinline__ void poseidon_permute_duo(uint64_t s[6], uint32_t h, 
             }
             const double y0 = fma(0.5, pa + qa, fma(d0, x0, int_dbl(tab.mid[q][h])));
             const double other = shfl_xor_d(y0);
-            const uint64_t y = pr_pow7(pr_reduce_split(dbl_int(h ? other : y0), dbl_int(h ? y0 : other)));
+            const uint64_t y = pr_pow7<true>(pr_reduce_split(dbl_int(h ? other : y0), dbl_int(h ? y0 : other)));
             const double yp = word_dbl(h ? (uint32_t)(y >> 32) : (uint32_t)y);
             const double g = fma(d0, x0, yp - y0);
             duo_rows<2>(u, w, o, tab.pair[q][h]);
@@ -1085,7 +1221,7 @@ __device__ __forceinline__ void poseidon_permute_duo(uint64_t s[6], uint32_t h, 
 // zero-pads); `active` pairs load and store, the others compute on zeros.
 // n must be the same for all pairs of a warp.
 __device__ __forceinline__ void poseidon_hash_one_duo(const uint64_t *in, uint32_t n, uint64_t *out, bool active,
-                                                      uint32_t h, const PoseidonTab &tab) {
+                                                      uint32_t h, const PoseidonGroupTab &tab) {
     if (n <= 4) {
         if (active && h == 0)
             for (uint32_t i = 0; i < 4; i++) out[i] = i < n ? in[i] : 0ull;
@@ -1139,7 +1275,7 @@ struct HexGroup : HexLanes {
     double p2[6], q2[6];  // row t of their squares
     double c0, c6;        // C e0 at rows t and t + 6
     double d0;            // the diagonal term on thread 0, else 0
-    __device__ __forceinline__ explicit HexGroup(const PoseidonTab &tab) : HexLanes() {
+    __device__ __forceinline__ explicit HexGroup(const PoseidonGroupTab &tab) : HexLanes() {
         const double *row = tab.rows[t];
 #pragma unroll
         for (int k = 0; k < 6; k++) {
@@ -1161,7 +1297,7 @@ __device__ __forceinline__ uint64_t shfl64(uint64_t v, uint32_t src) {
 // o0, o1: lanes t and t + 6 of the state (partially reduced, in and out).
 // Every lane of the warp must call this (shuffles over the full warp).
 __device__ __forceinline__ void poseidon_permute_hex(uint64_t &o0, uint64_t &o1, const HexGroup &g,
-                                                     const PoseidonTab &tab) {
+                                                     const PoseidonGroupTab &tab) {
     using C = PoseidonCirc;
     constexpr double d0 = (double)PoseidonMds::d0();
     o0 = pr_add_c(o0, tab.rc0[g.t]);
@@ -1348,7 +1484,7 @@ __device__ __forceinline__ void poseidon2_permute_hex(uint64_t &o0, uint64_t &o1
     }
 }
 
-__device__ __forceinline__ void permute_hex(uint64_t &o0, uint64_t &o1, const HexGroup &g, const PoseidonTab &tab) {
+__device__ __forceinline__ void permute_hex(uint64_t &o0, uint64_t &o1, const HexGroup &g, const PoseidonGroupTab &tab) {
     poseidon_permute_hex(o0, o1, g, tab);
 }
 __device__ __forceinline__ void permute_hex(uint64_t &o0, uint64_t &o1, const HexGroup2 &g, const Poseidon2Tab &tab) {

@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(256) merkle_top(uint64_t *__restrict__ digests
 
 // Copies a hasher's round tables into shared memory (all threads of the block).
 template <int H>
-__device__ __forceinline__ void load_tab(typename TabOf<H>::type &dst) {
+__device__ __forceinline__ void load_tab(GroupTabOf<H> &dst) {
     const uint64_t *g = reinterpret_cast<const uint64_t *>(global_tab<H>());
     uint64_t *d = reinterpret_cast<uint64_t *>(&dst);
     for (uint32_t k = threadIdx.x; k < sizeof(dst) / 8; k += blockDim.x) d[k] = g[k];
@@ -120,7 +120,7 @@ constexpr int kDuoThreads = 128;
 __global__ void __launch_bounds__(kDuoThreads) merkle_leaves_duo(const uint64_t *__restrict__ leaves,
                                                                  uint64_t n_leaves, uint32_t leaf_size,
                                                                  uint64_t *__restrict__ out, LeafMap map) {
-    __shared__ PoseidonTab tab;  // per-thread table indices: shared memory, not the constant bank
+    __shared__ PoseidonGroupTab tab;  // per-thread table indices: shared memory, not the constant bank
     load_tab<kPoseidon>(tab);
     const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
     const uint64_t first = (t >> 5) << 4;  // the warp's first hash
@@ -143,7 +143,7 @@ template <int H>
 __global__ void __launch_bounds__(kHexThreads) merkle_leaves_hex(const uint64_t *__restrict__ leaves,
                                                                  uint64_t n_leaves, uint32_t leaf_size,
                                                                  uint64_t *__restrict__ out, LeafMap map) {
-    __shared__ typename TabOf<H>::type tab;
+    __shared__ GroupTabOf<H> tab;
     load_tab<H>(tab);
     const HexOf<H> g(tab);
     const uint64_t first = ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5) * 5;
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(kHexThreads) merkle_leaves_hex(const uint64_t 
 template <int H>
 __global__ void __launch_bounds__(kHexThreads) merkle_level_hex(uint64_t *__restrict__ digests, uint32_t lg_w,
                                                                 uint64_t n_caps, uint64_t ds) {
-    __shared__ typename TabOf<H>::type tab;
+    __shared__ GroupTabOf<H> tab;
     load_tab<H>(tab);
     const HexOf<H> g(tab);
     const uint64_t w = 1ull << lg_w;
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(kHexThreads) merkle_level_hex(uint64_t *__rest
 template <int H>
 __global__ void __launch_bounds__(224) merkle_top_hex(uint64_t *__restrict__ digests, uint64_t *__restrict__ cap,
                                                        uint64_t ds, uint32_t w_top) {
-    __shared__ typename TabOf<H>::type tab;
+    __shared__ GroupTabOf<H> tab;
     load_tab<H>(tab);
     const HexOf<H> g(tab);
     const uint64_t sub = blockIdx.x;
