@@ -311,10 +311,15 @@ def merkle_tree(leaves, cap_height: int, hash_type: int = HashPoseidon, digests=
     assert leaves.dtype == torch.uint64 and leaves.is_cuda and leaves.is_contiguous() and leaves.dim() == 2
     n_leaves, w = leaves.shape
     n_digests, n_caps = merkle_sizes(n_leaves, cap_height)
+    # The tree writes every word, but for Keccak digests of leaves shorter than a digest and the one
+    # spare digest of a tree without levels; zeroing costs two launches.
+    written = w >= 4 or hash_type != HashKeccak
     if digests is None:
-        digests = torch.zeros((max(n_digests, 1), 4), dtype=torch.uint64, device=leaves.device)
+        new = torch.empty if written and n_digests else torch.zeros
+        digests = new((max(n_digests, 1), 4), dtype=torch.uint64, device=leaves.device)
     if cap is None:
-        cap = torch.zeros((n_caps, 4), dtype=torch.uint64, device=leaves.device)
+        new = torch.empty if written else torch.zeros
+        cap = new((n_caps, 4), dtype=torch.uint64, device=leaves.device)
     capi.check(capi.LIB.zk_merkle_async(digests.data_ptr(), cap.data_ptr(), leaves.data_ptr(), n_digests, n_caps,
                                         n_leaves, w, cap_height, hash_type, _stream_ptr(stream)))
     return digests, cap
@@ -396,8 +401,8 @@ def fri_commit(coeffs, rate_bits: int, arity_bits, cap_height: int, challenge, h
         view = leaves.view((n << rate_bits) >> ab, 2 << ab)
         dig, cap = merkle_tree(view, cap_height, hash_type, stream=stream)
         rnd = FriRound(view, dig, cap, ab, shift)
-        s = stream if stream is not None else torch.cuda.current_stream()
-        s.synchronize()
+        if stream is not None:
+            stream.synchronize()  # the copy below is ordered on the current stream only
         rnd.beta = challenge(i, cap.cpu().numpy())
         rounds.append(rnd)
         cur = fri_fold(cur, ab, rnd.beta, stream=stream)
