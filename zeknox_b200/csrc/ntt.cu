@@ -616,7 +616,7 @@ PassKernel rows_fixed_kernel(uint32_t l, uint32_t lg_t) {
 #define ZK_ROWS_CASE(LG_L, LG_T) \
     case ((LG_L) << 4 | (LG_T)): return ntt_rows_fixed<LG_L, LG_T, INV>;
     switch (l << 4 | lg_t) {
-        ZK_ROWS_CASE(6, 5) ZK_ROWS_CASE(7, 5) ZK_ROWS_CASE(8, 5) ZK_ROWS_CASE(9, 4) ZK_ROWS_CASE(10, 3)
+        ZK_ROWS_CASE(6, 5) ZK_ROWS_CASE(7, 5) ZK_ROWS_CASE(8, 5) ZK_ROWS_CASE(9, 3) ZK_ROWS_CASE(10, 2)
         ZK_ROWS_CASE(11, 2) ZK_ROWS_CASE(12, 1)
         default: return nullptr;
     }
@@ -1066,6 +1066,13 @@ static void launch_plan(const NttJob &j, const PassArgs &base, const Plan &plan,
                 a.lg_pre = lg - a.l;
                 a.lg_t = std::min<uint32_t>(ilog2_floor(kLinesElems) - a.l, plan.l[0]);
                 a.lg_t = std::min<uint32_t>(a.lg_t, 5);
+                // Lines of 512 and 1024 points: half as many per block, so half the
+                // shared memory and unrolled code (twice the resident blocks, and no
+                // waiting on instruction fetch, which was the first stall).  Row LDE
+                // 135 x 2^15 -> 2^18 0.497 -> 0.473 ms, 30 x 2^18 -> 2^20 0.601 -> 0.541.
+                // Shorter lines gain nothing (inverse 135 x 2^15: 95 -> 97 us), longer
+                // ones would store runs of one element.
+                if ((a.l == 9 || a.l == 10) && a.lg_t > 1) a.lg_t--;
                 a.src = scr;
                 a.src_poly_stride = N;
                 a.dst = j.dst + b0 * j.dst_stride;
