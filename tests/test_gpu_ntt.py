@@ -56,6 +56,19 @@ def test_lde_host_buffers(zk, oracle, lg_n, rate, batches):
     assert np.array_equal(out, oracle.batch_lde(x, lg_n, rate, batches))
 
 
+@pytest.mark.parametrize("lg_n,rate,batches", [(13, 1, 3), (15, 1, 2), (16, 1, 1), (17, 1, 1), (18, 2, 1), (19, 1, 1),
+                                               (20, 2, 1), (21, 1, 1), (23, 2, 1)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_lde_line_lengths_and_table_forms(zk, oracle, lg_n, rate, batches, inverse):
+    """Column passes of every line length, one and two zero-extension stages, one-load and two-level tables, and
+    (2^25 points) three passes."""
+    x = oracle.field_elems(2500 + lg_n, batches << lg_n)
+    d_out = _dev(np.zeros(batches << (lg_n + rate), dtype=np.uint64))
+    zk.lde_batch(0, d_out.data_ptr(), _dev(x).data_ptr(), lg_n, _cfg(zk, batches, rate, True, True, True),
+                 zk.INVERSE if inverse else zk.FORWARD)
+    assert np.array_equal(_host(d_out), oracle.batch_lde(x, lg_n, rate, batches, inverse=inverse, with_coset=True))
+
+
 @pytest.mark.parametrize("lg_n,rate,batches,inverse,coset", [
     (5, 2, 3, False, False), (5, 2, 3, True, True), (5, 2, 3, True, False), (12, 2, 2, True, True),
     (14, 3, 3, False, False), (14, 3, 3, True, True)])

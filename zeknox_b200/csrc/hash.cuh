@@ -39,7 +39,9 @@ namespace zk {
 //
 // Cost model behind the splits below (measured on the Poseidon leaf kernel): a
 // scheduler slot per instruction, two for an FP64 instruction and two for a
-// 32 x 32 -> 64-bit multiply; the kernels run at 90 % or more of that.
+// 32 x 32 -> 64-bit multiply; that kernel runs at 90 % of it (FP64 matrix
+// instructions take 11-12 slots next to integer work, for what is 8 FP64
+// instructions' worth of products, a quarter of them padding).
 __host__ __device__ constexpr uint64_t cx_canon(uint64_t a) { return a >= ZK_P ? a - ZK_P : a; }
 __host__ __device__ constexpr uint64_t cx_add_mod(uint64_t a, uint64_t b) {  // a, b < p
     return a >= ZK_P - b ? a - (ZK_P - b) : a + b;

@@ -439,16 +439,14 @@ using PassKernel = void (*)(PassArgs);
 
 // The column pass (kind 0) of ntt_pass_kernel with the line length (2^LG_L),
 // lines per block (2^LG_T) and non-zero prefix of every line (2^LV, LV ==
-// LG_L: no zero extension) fixed at compile time, for launches with the
-// one-load twiddle table and, when there is a coset, the one-load coset table
-// (transforms of up to 2^20 points).  Thread t's elements are t + 256 j: its
-// line (t mod T) is fixed, and its element and output positions step by
-// constants.
+// LG_L: no zero extension) fixed at compile time.  Thread t's elements are
+// t + 256 j: its line (t mod T) is fixed, and its element and output positions
+// step by constants.  Twiddles and coset powers come from the one-load tables
+// where there are any (up to 2^20 points), else from the two-level ones.
 template <int LG_L, int LG_T, int LV, bool INV>
 __global__ void __launch_bounds__(kNttThreads) ntt_column_fixed(PassArgs a) {
     constexpr uint32_t L = 1u << LG_L, T = 1u << LG_T, TP = T > 1 ? T + 1 : 1, RR = LG_L - LV;
-    static_assert(RR == 0 || RR >= 2, "a one-stage zero extension takes the generic pass");
-    static_assert(T <= kNttThreads && (T << LG_L) % kNttThreads == 0, "block elements: a multiple of the threads");
+    static_assert(T <= kNttThreads && (RR >= 2 || (T << LV) % kNttThreads == 0), "block elements: a multiple of the threads");
     extern __shared__ uint64_t smem[];
     uint64_t *tw = smem;  // omega_L^e, e < L
     uint64_t *sm = smem + L;
@@ -466,7 +464,8 @@ __global__ void __launch_bounds__(kNttThreads) ntt_column_fixed(PassArgs a) {
     const uint64_t i0 = base + r;  // index within the polynomial of the line's element 0
     const uint32_t e0 = threadIdx.x >> LG_T;
     constexpr uint32_t DE = kNttThreads >> LG_T;  // element step between j and j + 1
-    const uint64_t *pre = a.pre_full;
+    const bool coset = a.pre_lo != nullptr;
+    const uint64_t *pre = coset ? a.pre_full : nullptr;
     __syncthreads();  // the twiddle table, read by the replication below
     if constexpr (RR >= 2) {
         // inputs (line block 1) and coset powers (line block 2) staged with asynchronous copies;
@@ -493,12 +492,33 @@ __global__ void __launch_bounds__(kNttThreads) ntt_column_fixed(PassArgs a) {
                 if (i < a.n_valid) {
                     v = nt_canon(sm[((1u << LV) + e) * TP + t]);
                     if (pre) v = nt_mul(v, sm[((2u << LV) + e) * TP + t]);
+                    else if (coset) v = nt_mul(v, pow2l(a.pre_lo, a.pre_hi, a.pre_h, i));
                 }
                 sm[e * TP + t] = v;
 #pragma unroll
                 for (uint32_t b = 1; b < (1u << RR); b++)
                     sm[((b << LV) + e) * TP + t] = nt_mul(v, tw[(e * brev_const(b, RR)) & (L - 1)]);
             }
+        }
+    } else if constexpr (RR == 1) {
+        // one zero-extension stage: the line's upper half is the lower one twiddled
+        constexpr uint32_t NE = (T << LV) / kNttThreads;
+        uint64_t v[NE], c[NE];
+#pragma unroll
+        for (uint32_t j = 0; j < NE; j++) {  // all of a thread's loads in flight
+            const uint64_t i = i0 + ((uint64_t)(e0 + j * DE) << lg_s);
+            v[j] = i < a.n_valid ? src[(uint64_t)(e0 + j * DE) << lg_s] : 0;
+            c[j] = pre && i < a.n_valid ? __ldg(pre + i) : 0;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < NE; j++) {
+            const uint32_t e = e0 + j * DE;
+            const uint64_t i = i0 + ((uint64_t)e << lg_s);
+            v[j] = nt_canon(v[j]);
+            if (pre) v[j] = nt_mul(v[j], c[j]);
+            else if (coset && i < a.n_valid) v[j] = nt_mul(v[j], pow2l(a.pre_lo, a.pre_hi, a.pre_h, i));
+            sm[e * TP + t] = v[j];
+            sm[((1u << LV) + e) * TP + t] = nt_mul(v[j], tw[e]);
         }
     } else {
 #pragma unroll
@@ -508,7 +528,7 @@ __global__ void __launch_bounds__(kNttThreads) ntt_column_fixed(PassArgs a) {
             uint64_t v = 0;
             if (i < a.n_valid) {
                 v = nt_canon(src[(uint64_t)e << lg_s]);
-                if (pre) v = nt_mul(v, __ldg(pre + i));
+                if (coset) v = nt_mul(v, pow_at(pre, a.pre_lo, a.pre_hi, a.pre_h, i));
             }
             sm[e * TP + t] = v;
         }
@@ -517,19 +537,18 @@ __global__ void __launch_bounds__(kNttThreads) ntt_column_fixed(PassArgs a) {
     // Store with the inter-pass twiddle w_N^(r k Q).  One table load per element
     // made the L1 data path the pass's busiest unit (a warp's 32 exponents lie in
     // 32 sectors), so each thread loads its first two values and the step and
-    // goes on by one product per element, two chains (the table has N <= 2^20
-    // entries, so exponents wrap mod 2^32 harmlessly).  Commit 135 x 2^15, whole
-    // call: 3.74 -> 3.65 ms.
+    // goes on by one product per element, two chains (N divides 2^32, so exponents
+    // wrap harmlessly).  Commit 135 x 2^15, whole call: 3.74 -> 3.65 ms.
     constexpr uint32_t PER = (T << LG_L) / kNttThreads, kChains = PER >= 2 ? 2 : 1;
     const uint32_t nmask = (uint32_t)((1ull << a.lg_n) - 1);
     const uint32_t krt = __brev(e0) >> (32 - LG_L);  // rev(k) of the first k = e0
     const uint32_t rk0 = (uint32_t)r * e0, rdk = (uint32_t)r * DE;
     const uint32_t lg_pre = a.lg_pre;
-    const uint64_t *twf = a.tw_full;
+    auto root = [&](uint32_t e) { return pow_at(a.tw_full, a.tw_lo, a.tw_hi, a.tw_h, (e << lg_pre) & nmask); };
     uint64_t twk[kChains];
 #pragma unroll
-    for (uint32_t m = 0; m < kChains; m++) twk[m] = __ldg(twf + (((rk0 + m * rdk) << lg_pre) & nmask));
-    const uint64_t stp = __ldg(twf + (((kChains * rdk) << lg_pre) & nmask));
+    for (uint32_t m = 0; m < kChains; m++) twk[m] = root(rk0 + m * rdk);
+    const uint64_t stp = root(kChains * rdk);
 #pragma unroll
     for (uint32_t m = 0; m < PER; m++) {
         const uint32_t k = e0 + m * DE;
@@ -545,12 +564,11 @@ template <bool INV>
 PassKernel column_fixed_kernel(uint32_t l, uint32_t lg_t, uint32_t lv) {
 #define ZK_COLUMN_CASES(LG_L, LG_T)                                                        \
     case ((LG_L) << 8 | (LG_T) << 4 | 0): return ntt_column_fixed<LG_L, LG_T, LG_L, INV>;      \
+    case ((LG_L) << 8 | (LG_T) << 4 | 1): return ntt_column_fixed<LG_L, LG_T, LG_L - 1, INV>;  \
     case ((LG_L) << 8 | (LG_T) << 4 | 2): return ntt_column_fixed<LG_L, LG_T, LG_L - 2, INV>;  \
     case ((LG_L) << 8 | (LG_T) << 4 | 3): return ntt_column_fixed<LG_L, LG_T, LG_L - 3, INV>;
     if (lv > l) return nullptr;
     switch (l << 8 | lg_t << 4 | (l - lv)) {
-        ZK_COLUMN_CASES(7, 5) ZK_COLUMN_CASES(8, 5) ZK_COLUMN_CASES(9, 4) ZK_COLUMN_CASES(10, 3)
-        ZK_COLUMN_CASES(11, 2) ZK_COLUMN_CASES(12, 1)
         ZK_COLUMN_CASES(7, 4) ZK_COLUMN_CASES(8, 4) ZK_COLUMN_CASES(9, 3) ZK_COLUMN_CASES(10, 2)
         ZK_COLUMN_CASES(11, 1) ZK_COLUMN_CASES(12, 0)
         default: return nullptr;
@@ -857,7 +875,7 @@ void launch_pass(const PassArgs &a, uint64_t groups, cudaStream_t s, bool after_
     }
     require(groups < (1ull << 31), "transform too large for one launch");
     PassKernel kern = a.inverse ? ntt_pass_kernel<true> : ntt_pass_kernel<false>;
-    if (a.kind == 0 && a.tw_full && (a.pre_full || !a.pre_lo) && fixed_passes_enabled()) {
+    if (a.kind == 0 && fixed_passes_enabled()) {
         // the compile-time column pass, when this shape has one (lv as the kernel computes it)
         const uint64_t S = 1ull << a.lg_s, L = 1ull << a.l;
         uint32_t lv = a.l;
@@ -1019,13 +1037,11 @@ static void launch_plan(const NttJob &j, const PassArgs &base, const Plan &plan,
                 a.lg_pre = lg - a.l - lg_s;
                 a.lg_t = std::min<uint32_t>(ilog2_floor(kLinesElems) - a.l, lg_s);
                 a.lg_t = std::min<uint32_t>(a.lg_t, 5);
-                // With the one-load twiddle table (up to 2^20 points, the compile-time
-                // column kernels) half as many lines per block: half the shared
-                // memory, so more resident blocks hide the loads.  Measured, LDE to
-                // leaves: 135 x 2^15 -> 2^18 0.645 -> 0.625 ms, 64 x 2^17 -> 2^19
-                // 0.741 -> 0.676, 16 x 2^12 -> 2^15 0.026 -> 0.020; without the table
-                // (the generic pass) 300 x 2^19 -> 2^22 got slower (35.1 -> 36.7).
-                if (base.tw_full && a.lg_t > 0) a.lg_t--;
+                // Half as many lines per block as shared memory would hold: more
+                // resident blocks hide the loads.  Measured, LDE to leaves: 135 x 2^15 ->
+                // 2^18 0.645 -> 0.625 ms, 64 x 2^17 -> 2^19 0.741 -> 0.676, 16 x 2^12 ->
+                // 2^15 0.026 -> 0.020.
+                if (a.lg_t > 0) a.lg_t--;
                 if (p == 0) {
                     a.src = j.src + b0 * j.src_stride;
                     a.src_poly_stride = j.src_stride;
