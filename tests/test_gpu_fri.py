@@ -101,6 +101,31 @@ def test_fri_commit_matches_oracle(zk, oracle, lg_n, rate, arities, cap_h, ht):
     assert np.array_equal(_host(com.final_poly), final)
 
 
+def test_fri_commit_on_a_side_stream(zk, oracle):
+    """Rounds and openings on a given stream, while the current one has work of its own."""
+    import torch
+
+    lg_n, rate, arities, cap_h = 10, 3, [4, 3, 2], 2
+    n = 1 << lg_n
+    c = oracle.field_elems(9350, 2 * n).reshape(2, n)
+    rounds, final = oracle.fri_commit(c, rate, arities, cap_h, _challenge, 0)
+    d, side = _dev(c), torch.cuda.Stream()
+    x = torch.ones(4096, 4096, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(50):
+        x = x @ x * 2.0**-12
+    com = zk.fri_commit(d, rate, arities, cap_h, _challenge, stream=side)
+    q = torch.tensor([0, 5, (n << rate) - 1])
+    opened = zk.fri_open(com, q, stream=side)
+    opened_d = zk.merkle_open(com.rounds[0].leaves, com.rounds[0].digests, cap_h, (q >> 4).to("cuda"), stream=side)
+    torch.cuda.synchronize()
+    for g, w, (rows, _), sh in zip(com.rounds, rounds, opened, (4, 7, 9)):
+        assert np.array_equal(_host(g.leaves), w["leaves"]) and np.array_equal(_host(g.cap).reshape(-1), w["cap"])
+        assert np.array_equal(_host(g.digests).reshape(-1)[:w["digests"].size], w["digests"])
+        assert np.array_equal(_host(rows), w["leaves"][q.numpy() >> sh])
+    assert np.array_equal(_host(opened_d[0]), _host(opened[0][0])) and np.array_equal(_host(com.final_poly), final)
+
+
 def _check_rounds(oracle, com, rate_bits, rows_per_round, positions):
     """The FRI verifier's fold relation on the given leaf positions of every round."""
     for i, rnd in enumerate(com.rounds):

@@ -129,6 +129,29 @@ def test_edge_words_vs_oracle(zk, oracle, ht, nl, ls, ch):
     assert np.array_equal(c, c2) and np.array_equal(d, d2)
 
 
+@pytest.mark.parametrize("ht,ls", [(1, 3), (1, 17), (0, 9)])
+def test_side_stream_with_work_pending_on_the_current_one(zk, oracle, ht, ls):
+    """Outputs of a tree on another stream are no block that work pending on the current stream still writes."""
+    import torch
+
+    nl, ch = 4096, 2
+    leaves = oracle.field_elems(77 + ht * 10 + ls, nl * ls)
+    d2, c2 = oracle.merkle_fill(leaves, ls, ch, ht)
+    d_leaves = _dev(leaves.reshape(nl, ls))
+    side = torch.cuda.Stream()
+    x = torch.ones(4096, 4096, device="cuda")
+    torch.cuda.synchronize()
+    freed = [torch.empty((n, 4), dtype=torch.int64, device="cuda") for n in (2 * (nl - 4), 4)]
+    for _ in range(50):
+        x = x @ x * 2.0**-12  # a few tens of ms
+    for t in freed:
+        t.fill_(-1)
+    del t, freed
+    dig, cap = zk.merkle_tree(d_leaves, ch, ht, stream=side)
+    torch.cuda.synchronize()
+    assert np.array_equal(dig.cpu().numpy().reshape(-1), d2) and np.array_equal(cap.cpu().numpy().reshape(-1), c2)
+
+
 def test_cpu_entry_point(zk, oracle):
     """fill_digests_buf_linear_cpu: host buffers, same tree."""
     nl, ls, ch = 1024, 135, 4

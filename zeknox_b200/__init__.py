@@ -9,6 +9,8 @@ streams here.
 
 from __future__ import annotations
 
+import contextlib
+
 from . import capi
 from .capi import (  # noqa: F401
     FORWARD,
@@ -47,6 +49,36 @@ def _stream_ptr(stream) -> int:
     return int(s.cuda_stream)
 
 
+def _torch_stream(stream):
+    """`stream` as torch takes it: any object with a cuda_stream handle will do."""
+    import torch
+
+    return stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(int(stream.cuda_stream))
+
+
+def _on(stream):
+    """The current stream set to `stream` (None: as it is)."""
+    import torch
+
+    return contextlib.nullcontext() if stream is None else torch.cuda.stream(_torch_stream(stream))
+
+
+def _new(shape, device, stream, zero: bool = False):
+    """A uint64 tensor for work on `stream`.
+
+    torch hands a freed block out again in the order of the stream that it was
+    allocated on.  So it is allocated on `stream`: a block of the current stream
+    may still be in use by work pending there.  Once dropped, it is held until
+    the caller's stream is done with it too."""
+    import torch
+
+    with _on(stream):
+        t = (torch.zeros if zero else torch.empty)(shape, dtype=torch.uint64, device=device)
+    if stream is not None:
+        t.record_stream(torch.cuda.current_stream(device))
+    return t
+
+
 def lde(coeffs, rate_bits: int, *, inverse: bool = False, with_coset: bool = True, out=None, stream=None):
     """Coset LDE of the rows of a (B, 2^lg_n) uint64 CUDA tensor -> (B, 2^(lg_n+rate_bits)).
 
@@ -58,7 +90,7 @@ def lde(coeffs, rate_bits: int, *, inverse: bool = False, with_coset: bool = Tru
     lg_n = n.bit_length() - 1
     assert n == 1 << lg_n
     if out is None:
-        out = torch.empty((b, n << rate_bits), dtype=torch.uint64, device=coeffs.device)
+        out = _new((b, n << rate_bits), coeffs.device, stream)
     capi.check(capi.LIB.zk_lde_async(out.data_ptr(), coeffs.data_ptr(), lg_n, rate_bits, b, int(inverse),
                                      int(with_coset), _stream_ptr(stream)))
     return out
@@ -73,7 +105,7 @@ def transpose_rev(mat, out=None, stream=None):
     lg = n.bit_length() - 1
     assert n == 1 << lg
     if out is None:
-        out = torch.empty((n, b), dtype=torch.uint64, device=mat.device)
+        out = _new((n, b), mat.device, stream)
     capi.check(capi.LIB.zk_transpose_rev_async(out.data_ptr(), mat.data_ptr(), lg, b, _stream_ptr(stream)))
     return out
 
@@ -88,7 +120,7 @@ def lde_leaves(coeffs, rate_bits: int, out=None, stream=None):
     lg_n = n.bit_length() - 1
     assert n == 1 << lg_n
     if out is None:
-        out = torch.empty((n << rate_bits, b), dtype=torch.uint64, device=coeffs.device)
+        out = _new((n << rate_bits, b), coeffs.device, stream)
     capi.check(capi.LIB.zk_lde_leaves_async(out.data_ptr(), coeffs.data_ptr(), lg_n, rate_bits, b, _stream_ptr(stream)))
     return out
 
@@ -102,7 +134,7 @@ def lde_leaves_coset(coeffs, rate_bits: int, coset_gen: int, out=None, stream=No
     lg_n = n.bit_length() - 1
     assert n == 1 << lg_n
     if out is None:
-        out = torch.empty((n << rate_bits, b), dtype=torch.uint64, device=coeffs.device)
+        out = _new((n << rate_bits, b), coeffs.device, stream)
     capi.check(capi.LIB.zk_lde_leaves_coset_async(out.data_ptr(), coeffs.data_ptr(), lg_n, rate_bits, b,
                                                   coset_gen % P, _stream_ptr(stream)))
     return out
@@ -111,13 +143,11 @@ def lde_leaves_coset(coeffs, rate_bits: int, coset_gen: int, out=None, stream=No
 class CommitBuffers:
     """Device outputs of one commit: leaves (N, B), digests (2(N - 2^cap), 4), cap (2^cap, 4)."""
 
-    def __init__(self, n_leaves: int, width: int, cap_height: int, device="cuda"):
-        import torch
-
+    def __init__(self, n_leaves: int, width: int, cap_height: int, device="cuda", stream=None):
         nd, nc = merkle_sizes(n_leaves, cap_height)
-        self.leaves = torch.empty((n_leaves, width), dtype=torch.uint64, device=device)
-        self.digests = torch.empty((max(nd, 1), 4), dtype=torch.uint64, device=device)
-        self.cap = torch.empty((nc, 4), dtype=torch.uint64, device=device)
+        self.leaves = _new((n_leaves, width), device, stream)
+        self.digests = _new((max(nd, 1), 4), device, stream)
+        self.cap = _new((nc, 4), device, stream)
 
 
 def commit(coeffs, rate_bits: int, cap_height: int, hash_type: int = HashPoseidon, out: CommitBuffers | None = None,
@@ -126,7 +156,7 @@ def commit(coeffs, rate_bits: int, cap_height: int, hash_type: int = HashPoseido
     b, n = coeffs.shape
     lg_n = n.bit_length() - 1
     if out is None:
-        out = CommitBuffers(n << rate_bits, b, cap_height, coeffs.device)
+        out = CommitBuffers(n << rate_bits, b, cap_height, coeffs.device, stream)
     capi.check(capi.LIB.zk_commit_async(coeffs.data_ptr(), lg_n, rate_bits, b, cap_height, hash_type,
                                         out.leaves.data_ptr(), out.digests.data_ptr(), out.cap.data_ptr(),
                                         _stream_ptr(stream)))
@@ -315,11 +345,9 @@ def merkle_tree(leaves, cap_height: int, hash_type: int = HashPoseidon, digests=
     # spare digest of a tree without levels; zeroing costs two launches.
     written = w >= 4 or hash_type != HashKeccak
     if digests is None:
-        new = torch.empty if written and n_digests else torch.zeros
-        digests = new((max(n_digests, 1), 4), dtype=torch.uint64, device=leaves.device)
+        digests = _new((max(n_digests, 1), 4), leaves.device, stream, zero=not (written and n_digests))
     if cap is None:
-        new = torch.empty if written else torch.zeros
-        cap = new((n_caps, 4), dtype=torch.uint64, device=leaves.device)
+        cap = _new((n_caps, 4), leaves.device, stream, zero=not written)
     capi.check(capi.LIB.zk_merkle_async(digests.data_ptr(), cap.data_ptr(), leaves.data_ptr(), n_digests, n_caps,
                                         n_leaves, w, cap_height, hash_type, _stream_ptr(stream)))
     return digests, cap
@@ -334,11 +362,16 @@ def merkle_open(leaves, digests, cap_height: int, indices, stream=None):
 
     assert leaves.dtype == torch.uint64 and leaves.is_cuda and leaves.is_contiguous() and leaves.dim() == 2
     n_leaves, w = leaves.shape
-    idx = indices.to(device=leaves.device, dtype=torch.int64).contiguous().view(torch.uint64)
+    # A copy from the host is complete when it returns, whatever stream it took; work on `stream` does
+    # not hold it up.  A conversion on the device is only ordered where it runs.
+    with _on(stream if indices.is_cuda else None):
+        idx = indices.to(device=leaves.device, dtype=torch.int64).contiguous().view(torch.uint64)
+    if stream is not None:
+        idx.record_stream(_torch_stream(stream))
     q = idx.numel()
     depth = (n_leaves >> cap_height).bit_length() - 1
-    rows = torch.empty((q, w), dtype=torch.uint64, device=leaves.device)
-    sib = torch.empty((q, depth, 4), dtype=torch.uint64, device=leaves.device)
+    rows = _new((q, w), leaves.device, stream)
+    sib = _new((q, depth, 4), leaves.device, stream)
     capi.check(capi.LIB.zk_merkle_open_async(leaves.data_ptr(), digests.data_ptr(), n_leaves, w, cap_height,
                                              idx.data_ptr(), q, rows.data_ptr(), sib.data_ptr(), _stream_ptr(stream)))
     return rows, sib
@@ -357,7 +390,7 @@ def fri_fold(coeffs, arity_bits: int, beta, *, interleaved: bool = False, out=No
     n = coeffs.shape[0] if interleaved else coeffs.shape[1]
     assert coeffs.shape == ((n, 2) if interleaved else (2, n))
     if out is None:
-        out = torch.empty((2, n >> arity_bits), dtype=torch.uint64, device=coeffs.device)
+        out = _new((2, n >> arity_bits), coeffs.device, stream)
     capi.check(capi.LIB.zk_fri_fold_async(out.data_ptr(), coeffs.data_ptr(), n, arity_bits, int(beta[0]) % P,
                                           int(beta[1]) % P, int(interleaved), _stream_ptr(stream)))
     return out
@@ -390,8 +423,6 @@ def fri_commit(coeffs, rate_bits: int, arity_bits, cap_height: int, challenge, h
     (host callback, cap a (2^cap_height, 4) numpy array) returns beta; the
     coefficients are folded by beta (zk_fri_fold_async).  The final folded
     coefficients are returned on the device as `final_poly` (2, n / prod arity)."""
-    import torch
-
     assert coeffs.dim() == 2 and coeffs.shape[0] == 2
     cur = coeffs
     rounds = []
@@ -401,9 +432,9 @@ def fri_commit(coeffs, rate_bits: int, arity_bits, cap_height: int, challenge, h
         view = leaves.view((n << rate_bits) >> ab, 2 << ab)
         dig, cap = merkle_tree(view, cap_height, hash_type, stream=stream)
         rnd = FriRound(view, dig, cap, ab, shift)
-        if stream is not None:
-            stream.synchronize()  # the copy below is ordered on the current stream only
-        rnd.beta = challenge(i, cap.cpu().numpy())
+        with _on(stream):
+            cap_host = cap.cpu().numpy()  # waits for the round
+        rnd.beta = challenge(i, cap_host)
         rounds.append(rnd)
         cur = fri_fold(cur, ab, rnd.beta, stream=stream)
         shift = pow(shift, 1 << ab, P)
