@@ -171,6 +171,16 @@ def test_batch_ntt_forward_inverse(zk, oracle, lg, coset):
     assert np.array_equal(_host(d), oracle.batch_ntt(x, lg, True, batches, coset))
 
 
+@pytest.mark.parametrize("lg,batches", [(14, 3), (15, 5), (16, 2), (17, 9), (19, 2), (20, 1), (21, 1), (22, 1), (24, 1)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_batch_ntt_every_line_length(zk, oracle, lg, batches, inverse):
+    """Column passes without zero extension: lines of 2^7 to 2^12 points."""
+    x = oracle.field_elems(600 + lg, batches << lg)
+    d = _dev(x)
+    (zk.intt_batch if inverse else zk.ntt_batch)(0, d.data_ptr(), lg, _cfg(zk, batches, in_dev=True, out_dev=True))
+    assert np.array_equal(_host(d), oracle.batch_ntt(x, lg, inverse, batches))
+
+
 def test_ntt_three_pass_vs_oracle(zk, oracle):
     lg = 25  # three shared-memory passes
     x = oracle.field_elems(25, 1 << lg)

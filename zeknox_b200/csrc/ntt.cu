@@ -443,8 +443,21 @@ using PassKernel = void (*)(PassArgs);
 // t + 256 j: its line (t mod T) is fixed, and its element and output positions
 // step by constants.  Twiddles and coset powers come from the one-load tables
 // where there are any (up to 2^20 points), else from the two-level ones.
+//
+// Without zero extension a pass waits on its loads, so what counts is how many
+// blocks an SM holds.  The twiddle chains took lines of 512 and (forward) 1024
+// points past 64 registers, to 88 and 80, and from four blocks to two and three:
+// they are held to 64 (no spills).  Inverse 135 x 2^17 437 -> 352 us (396 with a
+// table load per element in place of the chains), 135 x 2^18 813 -> 633, 1 x 2^25
+// 1128 -> 951; forward 135 x 2^19 1428 -> 1339.  Forms that take no more than 64
+// are left alone: held to four blocks as well, they lost up to 2 % (inverse
+// 135 x 2^19 1330 -> 1354 us, 16 x 2^21 835 -> 845).
+template <int LG_L, int LV, bool INV>
+constexpr int column_blocks() {  // resident blocks to compile for; 0: no bound
+    return LV == LG_L && (LG_L == 9 || (LG_L == 10 && !INV)) ? 4 : 0;
+}
 template <int LG_L, int LG_T, int LV, bool INV>
-__global__ void __launch_bounds__(kNttThreads) ntt_column_fixed(PassArgs a) {
+__global__ void __launch_bounds__(kNttThreads, column_blocks<LG_L, LV, INV>()) ntt_column_fixed(PassArgs a) {
     constexpr uint32_t L = 1u << LG_L, T = 1u << LG_T, TP = T > 1 ? T + 1 : 1, RR = LG_L - LV;
     static_assert(T <= kNttThreads && (RR >= 2 || (T << LV) % kNttThreads == 0), "block elements: a multiple of the threads");
     extern __shared__ uint64_t smem[];
