@@ -63,10 +63,27 @@ def test_lde_line_lengths_and_table_forms(zk, oracle, lg_n, rate, batches, inver
     """Column passes of every line length, one and two zero-extension stages, one-load and two-level tables, and
     (2^25 points) three passes."""
     x = oracle.field_elems(2500 + lg_n, batches << lg_n)
-    d_out = _dev(np.zeros(batches << (lg_n + rate), dtype=np.uint64))
-    zk.lde_batch(0, d_out.data_ptr(), _dev(x).data_ptr(), lg_n, _cfg(zk, batches, rate, True, True, True),
+    d_in, d_out = _dev(x), _dev(np.zeros(batches << (lg_n + rate), dtype=np.uint64))
+    zk.lde_batch(0, d_out.data_ptr(), d_in.data_ptr(), lg_n, _cfg(zk, batches, rate, True, True, True),
                  zk.INVERSE if inverse else zk.FORWARD)
     assert np.array_equal(_host(d_out), oracle.batch_lde(x, lg_n, rate, batches, inverse=inverse, with_coset=True))
+
+
+@pytest.mark.parametrize("lg_n,rate,batches", [(9, 4, 3), (10, 5, 2), (14, 4, 2), (12, 6, 1), (17, 4, 1), (15, 6, 2),
+                                               (17, 5, 1), (18, 5, 1), (20, 4, 1)])
+@pytest.mark.parametrize("inverse,coset", [(False, True), (True, True), (False, False)])
+def test_lde_four_and_more_extension_stages(zk, oracle, lg_n, rate, batches, inverse, coset):
+    """Rates of 16 and more, whose column pass has no compiled form: below and above 2^20 points, each line length."""
+    x = oracle.field_elems(2600 + lg_n * 10 + rate, batches << lg_n)
+    d_in = _dev(x)
+    d_out = _dev(np.zeros(batches << (lg_n + rate), dtype=np.uint64))
+    zk.lde_batch(0, d_out.data_ptr(), d_in.data_ptr(), lg_n, _cfg(zk, batches, rate, True, True, coset),
+                 zk.INVERSE if inverse else zk.FORWARD)
+    want = oracle.batch_lde(x, lg_n, rate, batches, inverse=inverse, with_coset=coset)
+    assert np.array_equal(_host(d_out), want)
+    if coset and not inverse:  # and written as leaves
+        leaves = zk.lde_leaves(d_in.view(batches, -1), rate)
+        assert np.array_equal(_host(leaves).reshape(-1), oracle.transpose_rev(want, lg_n + rate, batches))
 
 
 @pytest.mark.parametrize("lg_n,rate,batches,inverse,coset", [

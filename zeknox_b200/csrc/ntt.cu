@@ -842,6 +842,15 @@ size_t pass_smem(uint32_t l, uint32_t lg_t) {
     return (size_t)(L + L * tp) * sizeof(uint64_t);
 }
 
+// log2 of the elements of a column pass's lines that can be non-zero (zero
+// extension), as the kernels compute it.
+uint32_t column_prefix_lg(const PassArgs &a) {
+    const uint64_t S = 1ull << a.lg_s, L = 1ull << a.l;
+    if (a.n_valid >= (L << a.lg_s) || a.lg_pre != 0) return a.l;
+    const uint64_t nz = (a.n_valid + S - 1) >> a.lg_s;
+    return nz <= 1 ? 0 : 64 - __builtin_clzll(nz - 1);
+}
+
 // after_pass: the previous launch on `s` is the pass before this one of the
 // same transform, so this pass may start while it drains (pdl.cuh).
 // ZK_NTT_GENERIC_PASSES=1 keeps the runtime-shaped pass kernels for every
@@ -889,13 +898,8 @@ void launch_pass(const PassArgs &a, uint64_t groups, cudaStream_t s, bool after_
     require(groups < (1ull << 31), "transform too large for one launch");
     PassKernel kern = a.inverse ? ntt_pass_kernel<true> : ntt_pass_kernel<false>;
     if (a.kind == 0 && fixed_passes_enabled()) {
-        // the compile-time column pass, when this shape has one (lv as the kernel computes it)
-        const uint64_t S = 1ull << a.lg_s, L = 1ull << a.l;
-        uint32_t lv = a.l;
-        if (a.n_valid < (L << a.lg_s) && a.lg_pre == 0) {
-            const uint64_t nz = (a.n_valid + S - 1) >> a.lg_s;
-            lv = nz <= 1 ? 0 : 64 - __builtin_clzll(nz - 1);
-        }
+        // the compile-time column pass, when this shape has one
+        const uint32_t lv = column_prefix_lg(a);
         PassKernel fixed = a.inverse ? column_fixed_kernel<true>(a.l, a.lg_t, lv)
                                      : column_fixed_kernel<false>(a.l, a.lg_t, lv);
         if (fixed) {
@@ -1055,11 +1059,6 @@ static void launch_plan(const NttJob &j, const PassArgs &base, const Plan &plan,
                 a.lg_pre = lg - a.l - lg_s;
                 a.lg_t = std::min<uint32_t>(ilog2_floor(kLinesElems) - a.l, lg_s);
                 a.lg_t = std::min<uint32_t>(a.lg_t, 5);
-                // Half as many lines per block as shared memory would hold: more
-                // resident blocks hide the loads.  Measured, LDE to leaves: 135 x 2^15 ->
-                // 2^18 0.645 -> 0.625 ms, 64 x 2^17 -> 2^19 0.741 -> 0.676, 16 x 2^12 ->
-                // 2^15 0.026 -> 0.020.
-                if (a.lg_t > 0) a.lg_t--;
                 if (p == 0) {
                     a.src = j.src + b0 * j.src_stride;
                     a.src_poly_stride = j.src_stride;
@@ -1070,6 +1069,19 @@ static void launch_plan(const NttJob &j, const PassArgs &base, const Plan &plan,
                     a.n_valid = N;
                     a.pre_lo = nullptr;
                 }
+                // Half as many lines per block as shared memory would hold: more resident
+                // blocks hide the loads.  Measured, LDE to leaves: 135 x 2^15 -> 2^18 0.645 ->
+                // 0.625 ms, 64 x 2^17 -> 2^19 0.741 -> 0.676, 16 x 2^12 -> 2^15 0.026 -> 0.020.
+                // Above 2^20 points (full -> half, us, four polynomials): 2^23 without zero
+                // extension 1804 -> 1176, 2^20 rate 1 -> 2^21 300 -> 211, three passes 2^22
+                // rate 3 -> 2^25 3631 -> 3151.  With two or three zero-extension stages, lines of
+                // 2^11 points would be 5 % faster full with several polynomials and up to 8 %
+                // slower with one (2^19 -> 2^22: 4 polynomials 370 / 388, one 114 / 105); of 2^12
+                // points it is even.  From four stages on (the runtime-shaped pass, which
+                // reads little) lines of 2^11 and 2^12 points stay full: 4 x 2^18 -> 2^23
+                // 889 against 995, 1 x 2^15 -> 2^21 to leaves 62 against 70 (two polynomials of
+                // 2^17 -> 2^21, the worst of 88 shapes: 91 against 89.5).
+                if (a.lg_t > 0 && !(a.l >= 11 && a.l - column_prefix_lg(a) >= 4)) a.lg_t--;
                 a.dst = scr;
                 a.dst_poly_stride = N;
                 a.post_lo = nullptr;
