@@ -206,6 +206,53 @@ def test_ntt_three_pass_vs_oracle(zk, oracle):
     assert np.array_equal(_host(d), oracle.batch_ntt(x, lg, False, 1, True))
 
 
+PLANS = """
+import sys
+import numpy as np, torch
+import zeknox_b200 as zk
+from oracle import oracle as O
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+for lg_n, rate, b in {shapes}:
+    lg = lg_n + rate
+    x = O.field_elems(2700 + lg, b << lg_n)
+    d = dev(x).view(b, -1)
+    for inverse, coset in [(False, True), (True, True), (False, False)][:({rows} and (1 if lg > 22 else 3))]:
+        got = zk.lde(d, rate, inverse=inverse, with_coset=coset).cpu().numpy().reshape(-1)
+        assert np.array_equal(got, O.batch_lde(x, lg_n, rate, b, inverse=inverse, with_coset=coset)), (lg_n, rate, inverse, coset)
+    leaves = zk.lde_leaves(d, rate).cpu().numpy().reshape(-1)
+    assert np.array_equal(leaves, O.transpose_rev(O.batch_lde(x, lg_n, rate, b), lg, b)), (lg_n, rate, "leaves")
+    if lg > 22:
+        continue
+    shifted = zk.lde_leaves_coset(d, rate, 7**16).cpu().numpy().reshape(-1)
+    want = O.transpose_rev(O.batch_lde(x, lg_n, rate, b, coset_gen=7**16), lg, b)
+    assert np.array_equal(shifted, want), (lg_n, rate, "shifted")
+print("equal")
+"""
+
+
+@pytest.mark.parametrize("env,shapes,rows", [
+    # three passes where a static plan takes two: the coset is applied once (2^20 points have it in one table)
+    ({"ZK_NTT_LEAVES_PASSES": "3"}, [(10, 3, 9), (14, 1, 3), (15, 3, 5), (17, 3, 2), (18, 2, 1), (19, 2, 1)], False),
+    ({"ZK_NTT_LEAVES_PASSES": "2"}, [(19, 3, 1), (20, 3, 2)], False),
+    # the runtime-shaped passes: columns, rows and leaves
+    ({"ZK_NTT_GENERIC_PASSES": "1"}, [(10, 3, 5), (12, 1, 9), (15, 3, 3), (17, 3, 1), (14, 4, 2), (20, 2, 1), (22, 3, 1)], True),
+    ({"ZK_NTT_GENERIC_PASSES": "1", "ZK_NTT_LEAVES_PASSES": "3"}, [(12, 2, 9), (17, 3, 2)], False)])
+def test_lde_plans_and_runtime_shaped_passes(oracle, env, shapes, rows):
+    """Plans and kernels that a shape does not take by itself, in a process of their own (the switches are read once)."""
+    import os
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    root = Path(__file__).resolve().parents[1]
+    r = subprocess.run([sys.executable, "-c", PLANS.format(shapes=shapes, rows=rows)], cwd=root, timeout=600,
+                       env={**os.environ, **env, "PYTHONPATH": str(root)}, capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip() == "equal", r.stdout + r.stderr
+
+
 def test_ntt_roundtrip_large(zk, oracle):
     # size-independent property at 2^26: iNTT(NTT(x)) == x
     lg, b = 26, 1

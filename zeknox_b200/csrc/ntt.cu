@@ -952,8 +952,20 @@ uint64_t tune_key(uint32_t lg, uint64_t batches) {
     return ((uint64_t)lg << 8) | cls;
 }
 
+// ZK_NTT_LEAVES_PASSES=2 or 3 fixes the number of passes of every LDE to
+// leaves that has more than one (same outputs; for comparing the plans, which
+// the tuner otherwise picks by time).
+int fixed_leaves_passes(uint32_t lg) {
+    static const int n = [] {
+        const char *e = getenv("ZK_NTT_LEAVES_PASSES");
+        return e && (e[0] == '2' || e[0] == '3') && !e[1] ? e[0] - '0' : 0;
+    }();
+    return lg <= 12 || (n == 2 && lg > 24) ? 0 : n;
+}
+
 LeavesChoice leaves_choice(uint32_t lg, uint64_t batches) {
     if (t_tune_override) return *t_tune_override;
+    if (const int n = fixed_leaves_passes(lg)) return LeavesChoice{(uint8_t)n, 3};
     std::lock_guard<std::mutex> g(g_tune_mu);
     auto it = g_tune.find(tune_key(lg, batches));
     return it == g_tune.end() ? LeavesChoice{} : it->second;
@@ -1067,7 +1079,7 @@ static void launch_plan(const NttJob &j, const PassArgs &base, const Plan &plan,
                     a.src = scr;
                     a.src_poly_stride = N;
                     a.n_valid = N;
-                    a.pre_lo = nullptr;
+                    a.pre_lo = a.pre_full = nullptr;
                 }
                 // Half as many lines per block as shared memory would hold: more resident
                 // blocks hide the loads.  Measured, LDE to leaves: 135 x 2^15 -> 2^18 0.645 ->
@@ -1102,7 +1114,7 @@ static void launch_plan(const NttJob &j, const PassArgs &base, const Plan &plan,
                 a.src_poly_stride = N;
                 a.dst = j.dst + b0;
                 a.leaf_stride = j.leaf_stride ? j.leaf_stride : j.batches;
-                a.pre_lo = nullptr;
+                a.pre_lo = a.pre_full = nullptr;
                 a.n_valid = N;
                 const uint64_t groups = ((nb + (1ull << a.lg_t) - 1) >> a.lg_t) << a.lg_pre;
                 launch_leaves_pass(a, groups, s);
@@ -1123,7 +1135,7 @@ static void launch_plan(const NttJob &j, const PassArgs &base, const Plan &plan,
                 a.src_poly_stride = N;
                 a.dst = j.dst + b0 * j.dst_stride;
                 a.dst_poly_stride = j.dst_stride;
-                a.pre_lo = nullptr;
+                a.pre_lo = a.pre_full = nullptr;
                 a.n_valid = N;
                 const uint64_t groups = nb << (a.lg_pre - a.lg_t);
                 launch_pass(a, groups, s, true);
