@@ -4,7 +4,7 @@
 // are bit-identical to zeknox's gl64_t (native/ff/gl64_t.cuh:93-369) and
 // cpp_gl64_t (native/ff/goldilocks.hpp:139-177), whose outputs are canonical
 // for canonical inputs.  The 64x64 -> 128-bit product is formed from 32-bit
-// IMAD chains; the reduction uses 2^64 = 2^32 - 1 and 2^96 = -1 (mod p).
+// IMAD chains; the reductions use 2^64 = 2^32 - 1 and 2^96 = -1 (mod p).
 #pragma once
 #include <stdint.h>
 
@@ -30,45 +30,6 @@ __device__ __forceinline__ uint64_t gl_add(uint64_t a, uint64_t b) {
         : "=l"(s), "=l"(t), "=r"(c)
         : "l"(a), "l"(b), "l"(ZK_EPS));
     return c ? t : s;
-}
-
-// a - b mod p for a, b < p: on borrow add p, i.e. subtract EPS.
-__device__ __forceinline__ uint64_t gl_sub(uint64_t a, uint64_t b) {
-    uint64_t d;
-    uint32_t bw;
-    asm("{\n\t"
-        "sub.cc.u64 %0, %2, %3;\n\t"
-        "subc.u32 %1, 0, 0;\n\t"
-        "}"
-        : "=l"(d), "=r"(bw)
-        : "l"(a), "l"(b));
-    return bw ? d - ZK_EPS : d;
-}
-
-// Reduce the 128-bit value (hi, lo) to canonical form.
-// x = lo + 2^64 (hl + 2^32 hh) = lo - hh + hl (2^32 - 1)  (mod p).
-__device__ __forceinline__ uint64_t gl_reduce128(uint64_t lo, uint64_t hi) {
-    uint32_t hl = (uint32_t)hi, hh = (uint32_t)(hi >> 32);
-    uint64_t t0;
-    uint32_t bw;
-    asm("{\n\t"
-        "sub.cc.u64 %0, %2, %3;\n\t"
-        "subc.u32 %1, 0, 0;\n\t"
-        "}"
-        : "=l"(t0), "=r"(bw)
-        : "l"(lo), "l"((uint64_t)hh));
-    if (bw) t0 -= ZK_EPS;                      // t0 in [p - 2^32 + 1, p) after a borrow
-    uint64_t t1 = ((uint64_t)hl << 32) - hl;   // hl * EPS <= p - 2^32
-    uint64_t r;
-    uint32_t c;
-    asm("{\n\t"
-        "add.cc.u64 %0, %2, %3;\n\t"
-        "addc.u32 %1, 0, 0;\n\t"
-        "}"
-        : "=l"(r), "=r"(c)
-        : "l"(t0), "l"(t1));
-    if (c) r += ZK_EPS;                        // cannot carry again: r < p - 2^32 here
-    return r >= ZK_P ? r - ZK_P : r;
 }
 
 // Full 64 x 64 -> 128-bit product from 32-bit limbs.
@@ -99,23 +60,6 @@ __device__ __forceinline__ uint64_t pr_mul(uint64_t a, uint64_t b);
 // Canonical product: the partially reduced product (below) then one
 // conditional subtraction.
 __device__ __forceinline__ uint64_t gl_mul(uint64_t a, uint64_t b) { return gl_canon_fwd(pr_mul(a, b)); }
-
-__device__ __forceinline__ uint64_t gl_sqr(uint64_t a) { return gl_mul(a, a); }
-
-// Reduce a value below 2^96 held as (lo, hi32): lo + hi32 * EPS (mod p).
-__device__ __forceinline__ uint64_t gl_reduce96(uint64_t lo, uint32_t hi32) {
-    uint64_t t1 = ((uint64_t)hi32 << 32) - hi32;  // hi32 * EPS
-    uint64_t r;
-    uint32_t c;
-    asm("{\n\t"
-        "add.cc.u64 %0, %2, %3;\n\t"
-        "addc.u32 %1, 0, 0;\n\t"
-        "}"
-        : "=l"(r), "=r"(c)
-        : "l"(lo), "l"(t1));
-    if (c) r += ZK_EPS;  // lo + t1 - 2^64 < 2^64 - 2^32, so this cannot carry
-    return r >= ZK_P ? r - ZK_P : r;
-}
 
 // Canonical representative of an arbitrary u64.
 __device__ __forceinline__ uint64_t gl_canon(uint64_t x) { return x >= ZK_P ? x - ZK_P : x; }

@@ -76,8 +76,8 @@ __global__ void __launch_bounds__(kLeafThreads) merkle_level(uint64_t *__restric
 // One block per subtree: the levels of width w_top, w_top/2, ..., 1 (the cap),
 // one node per thread, __syncthreads between levels.  These levels are few
 // nodes each, so every one costs about one permutation's latency: the block
-// copies its hasher's round tables into shared memory first and uses the
-// 12-lanes-at-once S-box.
+// copies its hasher's round tables into shared memory first.  For the hashers
+// without a form on several threads (Keccak, Monolith).
 template <int H>
 __global__ void __launch_bounds__(256) merkle_top(uint64_t *__restrict__ digests, uint64_t *__restrict__ cap,
                                                    uint64_t ds, uint32_t w_top) {
@@ -98,8 +98,8 @@ __global__ void __launch_bounds__(256) merkle_top(uint64_t *__restrict__ digests
         if (i < w) {
             const uint64_t *c = base + 4 * (2 * w - 2 + 2 * i);  // children 2i, 2i+1 of the level of width 2w
             uint64_t *o = w >= 2 ? base + 4 * (w - 2 + i) : cap + 4 * sub;
-            if constexpr (sizeof(Tab) >= 8) hash_two<H, 12>(c, c + 4, o, tab);
-            else hash_two<H, 12>(c, c + 4, o);
+            if constexpr (sizeof(Tab) >= 8) hash_two<H>(c, c + 4, o, tab);
+            else hash_two<H>(c, c + 4, o);
         }
         __syncthreads();
     }

@@ -459,7 +459,8 @@ constexpr int column_blocks() {  // resident blocks to compile for; 0: no bound
 template <int LG_L, int LG_T, int LV, bool INV>
 __global__ void __launch_bounds__(kNttThreads, column_blocks<LG_L, LV, INV>()) ntt_column_fixed(PassArgs a) {
     constexpr uint32_t L = 1u << LG_L, T = 1u << LG_T, TP = T > 1 ? T + 1 : 1, RR = LG_L - LV;
-    static_assert(T <= kNttThreads && (RR >= 2 || (T << LV) % kNttThreads == 0), "block elements: a multiple of the threads");
+    constexpr uint32_t NE = (T << LV) / kNttThreads;  // non-zero elements per thread
+    static_assert(T <= kNttThreads && (T << LV) % kNttThreads == 0, "block elements: a multiple of the threads");
     extern __shared__ uint64_t smem[];
     uint64_t *tw = smem;  // omega_L^e, e < L
     uint64_t *sm = smem + L;
@@ -483,39 +484,33 @@ __global__ void __launch_bounds__(kNttThreads, column_blocks<LG_L, LV, INV>()) n
     if constexpr (RR >= 2) {
         // inputs (line block 1) and coset powers (line block 2) staged with asynchronous copies;
         // each thread reads back only the slots it staged, before its replication overwrites them
-        constexpr uint32_t NE = (T << LV) < kNttThreads ? 1 : (T << LV) / kNttThreads;
-        if ((T << LV) >= kNttThreads || threadIdx.x < (T << LV)) {
 #pragma unroll
-            for (uint32_t j = 0; j < NE; j++) {
-                const uint32_t e = e0 + j * DE;
-                const uint64_t i = i0 + ((uint64_t)e << lg_s);
-                if (i < a.n_valid) {
-                    cp_async8(&sm[((1u << LV) + e) * TP + t], src + ((uint64_t)e << lg_s));
-                    if (pre) cp_async8(&sm[((2u << LV) + e) * TP + t], pre + i);
-                }
+        for (uint32_t j = 0; j < NE; j++) {
+            const uint32_t e = e0 + j * DE;
+            const uint64_t i = i0 + ((uint64_t)e << lg_s);
+            if (i < a.n_valid) {
+                cp_async8(&sm[((1u << LV) + e) * TP + t], src + ((uint64_t)e << lg_s));
+                if (pre) cp_async8(&sm[((2u << LV) + e) * TP + t], pre + i);
             }
         }
         cp_async_wait_all();
-        if ((T << LV) >= kNttThreads || threadIdx.x < (T << LV)) {
 #pragma unroll
-            for (uint32_t j = 0; j < NE; j++) {
-                const uint32_t e = e0 + j * DE;
-                const uint64_t i = i0 + ((uint64_t)e << lg_s);
-                uint64_t v = 0;
-                if (i < a.n_valid) {
-                    v = nt_canon(sm[((1u << LV) + e) * TP + t]);
-                    if (pre) v = nt_mul(v, sm[((2u << LV) + e) * TP + t]);
-                    else if (coset) v = nt_mul(v, pow2l(a.pre_lo, a.pre_hi, a.pre_h, i));
-                }
-                sm[e * TP + t] = v;
-#pragma unroll
-                for (uint32_t b = 1; b < (1u << RR); b++)
-                    sm[((b << LV) + e) * TP + t] = nt_mul(v, tw[(e * brev_const(b, RR)) & (L - 1)]);
+        for (uint32_t j = 0; j < NE; j++) {
+            const uint32_t e = e0 + j * DE;
+            const uint64_t i = i0 + ((uint64_t)e << lg_s);
+            uint64_t v = 0;
+            if (i < a.n_valid) {
+                v = nt_canon(sm[((1u << LV) + e) * TP + t]);
+                if (pre) v = nt_mul(v, sm[((2u << LV) + e) * TP + t]);
+                else if (coset) v = nt_mul(v, pow2l(a.pre_lo, a.pre_hi, a.pre_h, i));
             }
+            sm[e * TP + t] = v;
+#pragma unroll
+            for (uint32_t b = 1; b < (1u << RR); b++)
+                sm[((b << LV) + e) * TP + t] = nt_mul(v, tw[(e * brev_const(b, RR)) & (L - 1)]);
         }
     } else if constexpr (RR == 1) {
         // one zero-extension stage: the line's upper half is the lower one twiddled
-        constexpr uint32_t NE = (T << LV) / kNttThreads;
         uint64_t v[NE], c[NE];
 #pragma unroll
         for (uint32_t j = 0; j < NE; j++) {  // all of a thread's loads in flight
@@ -535,7 +530,7 @@ __global__ void __launch_bounds__(kNttThreads, column_blocks<LG_L, LV, INV>()) n
         }
     } else {
 #pragma unroll
-        for (uint32_t j = 0; j < (T << LG_L) / kNttThreads; j++) {
+        for (uint32_t j = 0; j < NE; j++) {
             const uint32_t e = e0 + j * DE;
             const uint64_t i = i0 + ((uint64_t)e << lg_s);
             uint64_t v = 0;
