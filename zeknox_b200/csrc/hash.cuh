@@ -284,9 +284,9 @@ static_assert(diag_only_lane0(), "the MDS layer below assumes diag(d, 0, ..., 0)
 // C^2 has row sums of 2^16; those of C^3 are 2^24, and with halves of 2^33 only
 // its entries less their common part kappa / 2 stay exact (sums below 2^53):
 // kappa / 2 times the sum of the lanes is formed mod p and added to every row.
-// One thread per hash takes three rounds at a time (rounds 4-24, and 25 alone);
-// the forms on several threads take two, whose dependent chain is the same
-// length per round but whose tables fit their shared memory copies better.
+// One thread per hash, bound by issue slots, takes three rounds at a time
+// (rounds 4-24, and 25 alone); the forms on several threads, bound by latency,
+// take two, whose dependent chain is the same length per round.
 struct PoseidonTab {          // one thread per hash
     uint64_t full[9][2][12];  // layers of rounds 0-3 and 25-29 (no constants after 29)
     uint64_t trip[7][2][12];  // layers of rounds (4, 5, 6) .. (22, 23, 24)
@@ -301,7 +301,7 @@ struct PoseidonGroupTab {      // several threads per hash
     // the six-thread form's rows t of A + B and A - B (for C and C^2), and C e0 at rows t and t + 6
     double rows[6][26];
 };
-constexpr uint64_t kFullBias = 1ull << 40;  // above the w offset of C: 113 * 2^31
+constexpr uint64_t kFullBias = 1ull << 40;  // above the w offset of C: 34 * 2^31
 constexpr uint64_t kPairBias = 1ull << 48;  // above 41 * 2^42 of -g and the w offset of C^2
 constexpr uint64_t kTripBias = 1ull << 49;  // above 2^33 times the negative entries of (C^3 - kappa / 2)
 struct Vec12 {
@@ -583,9 +583,9 @@ __device__ __forceinline__ void poseidon2_permute(uint64_t s[12], const Poseidon
 
 // --------------------------------------------------------------- Keccak
 // Keccak-f on 32-bit halves with each three-input operation written as one
-// lop3 and each rotation as two funnel shifts.  Bound by the ALU pipe (97 %
-// busy): from 64-bit words the compiler made about 220 ALU instructions and 28
-// moves a round where 180 do.  Tree 2^18 x 135: 0.771 -> 0.645 ms.
+// lop3 and each rotation as two funnel shifts: 180 operations a round (theta
+// 80, rho 48, chi 50, iota 2), all on the ALU pipe, which bounds it (97 % busy
+// already from 64-bit words).  Tree 2^18 x 135: 0.771 -> 0.645 ms.
 __device__ __forceinline__ uint32_t xor3(uint32_t a, uint32_t b, uint32_t c) {
     uint32_t r;
     asm("lop3.b32 %0, %1, %2, %3, 0x96;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
@@ -736,8 +736,9 @@ __device__ __forceinline__ void monolith_permute(uint64_t s[12], const MonolithT
 // below r plus the product over R, and the state elements that a partial round
 // adds to grow by less than 1.1 r in each of the 60 rounds, to below 2^260.
 // Products on carry chains of 32-bit limbs, the form before this one, left
-// each warp waiting on its chain.  Trees of 135-word leaves: 8192 leaves 27.2 ->
-// 12.5 ms, 65536 leaves 51.7 -> 33.8 ms.
+// each warp waiting on its chain.  Trees of 135-word leaves, one thread per hash
+// throughout: 8192 leaves 27.2 -> 12.5 ms, 65536 leaves 51.7 -> 33.8 ms (10.0 and
+// 31.7 with the narrow levels on five threads, end of file).
 constexpr int kBnL = 9;
 constexpr uint32_t kBnMask = (1u << 29) - 1;
 struct Fr {
