@@ -56,15 +56,18 @@ def _torch_stream(stream):
     return stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(int(stream.cuda_stream))
 
 
+_HERE = contextlib.nullcontext()
+
+
 def _on(stream):
-    """The current stream set to `stream` (None: as it is)."""
+    """The current stream set to `stream`."""
     import torch
 
-    return contextlib.nullcontext() if stream is None else torch.cuda.stream(_torch_stream(stream))
+    return torch.cuda.stream(_torch_stream(stream))
 
 
-def _new(shape, device, stream, zero: bool = False):
-    """A uint64 tensor for work on `stream`.
+def _on_stream(make, stream):
+    """`make` (torch.empty or torch.zeros) for a tensor that work on `stream` uses.
 
     torch hands a freed block out again in the order of the stream that it was
     allocated on.  So it is allocated on `stream`: a block of the current stream
@@ -72,11 +75,13 @@ def _new(shape, device, stream, zero: bool = False):
     the caller's stream is done with it too."""
     import torch
 
-    with _on(stream):
-        t = (torch.zeros if zero else torch.empty)(shape, dtype=torch.uint64, device=device)
-    if stream is not None:
+    def new(shape, *, dtype, device):
+        with _on(stream):
+            t = make(shape, dtype=dtype, device=device)
         t.record_stream(torch.cuda.current_stream(device))
-    return t
+        return t
+
+    return new
 
 
 def lde(coeffs, rate_bits: int, *, inverse: bool = False, with_coset: bool = True, out=None, stream=None):
@@ -90,7 +95,8 @@ def lde(coeffs, rate_bits: int, *, inverse: bool = False, with_coset: bool = Tru
     lg_n = n.bit_length() - 1
     assert n == 1 << lg_n
     if out is None:
-        out = _new((b, n << rate_bits), coeffs.device, stream)
+        new = torch.empty if stream is None else _on_stream(torch.empty, stream)
+        out = new((b, n << rate_bits), dtype=torch.uint64, device=coeffs.device)
     capi.check(capi.LIB.zk_lde_async(out.data_ptr(), coeffs.data_ptr(), lg_n, rate_bits, b, int(inverse),
                                      int(with_coset), _stream_ptr(stream)))
     return out
@@ -105,7 +111,8 @@ def transpose_rev(mat, out=None, stream=None):
     lg = n.bit_length() - 1
     assert n == 1 << lg
     if out is None:
-        out = _new((n, b), mat.device, stream)
+        new = torch.empty if stream is None else _on_stream(torch.empty, stream)
+        out = new((n, b), dtype=torch.uint64, device=mat.device)
     capi.check(capi.LIB.zk_transpose_rev_async(out.data_ptr(), mat.data_ptr(), lg, b, _stream_ptr(stream)))
     return out
 
@@ -120,7 +127,8 @@ def lde_leaves(coeffs, rate_bits: int, out=None, stream=None):
     lg_n = n.bit_length() - 1
     assert n == 1 << lg_n
     if out is None:
-        out = _new((n << rate_bits, b), coeffs.device, stream)
+        new = torch.empty if stream is None else _on_stream(torch.empty, stream)
+        out = new((n << rate_bits, b), dtype=torch.uint64, device=coeffs.device)
     capi.check(capi.LIB.zk_lde_leaves_async(out.data_ptr(), coeffs.data_ptr(), lg_n, rate_bits, b, _stream_ptr(stream)))
     return out
 
@@ -134,7 +142,8 @@ def lde_leaves_coset(coeffs, rate_bits: int, coset_gen: int, out=None, stream=No
     lg_n = n.bit_length() - 1
     assert n == 1 << lg_n
     if out is None:
-        out = _new((n << rate_bits, b), coeffs.device, stream)
+        new = torch.empty if stream is None else _on_stream(torch.empty, stream)
+        out = new((n << rate_bits, b), dtype=torch.uint64, device=coeffs.device)
     capi.check(capi.LIB.zk_lde_leaves_coset_async(out.data_ptr(), coeffs.data_ptr(), lg_n, rate_bits, b,
                                                   coset_gen % P, _stream_ptr(stream)))
     return out
@@ -144,10 +153,13 @@ class CommitBuffers:
     """Device outputs of one commit: leaves (N, B), digests (2(N - 2^cap), 4), cap (2^cap, 4)."""
 
     def __init__(self, n_leaves: int, width: int, cap_height: int, device="cuda", stream=None):
+        import torch
+
+        new = torch.empty if stream is None else _on_stream(torch.empty, stream)
         nd, nc = merkle_sizes(n_leaves, cap_height)
-        self.leaves = _new((n_leaves, width), device, stream)
-        self.digests = _new((max(nd, 1), 4), device, stream)
-        self.cap = _new((nc, 4), device, stream)
+        self.leaves = new((n_leaves, width), dtype=torch.uint64, device=device)
+        self.digests = new((max(nd, 1), 4), dtype=torch.uint64, device=device)
+        self.cap = new((nc, 4), dtype=torch.uint64, device=device)
 
 
 def commit(coeffs, rate_bits: int, cap_height: int, hash_type: int = HashPoseidon, out: CommitBuffers | None = None,
@@ -345,9 +357,13 @@ def merkle_tree(leaves, cap_height: int, hash_type: int = HashPoseidon, digests=
     # spare digest of a tree without levels; zeroing costs two launches.
     written = w >= 4 or hash_type != HashKeccak
     if digests is None:
-        digests = _new((max(n_digests, 1), 4), leaves.device, stream, zero=not (written and n_digests))
+        new = torch.empty if written and n_digests else torch.zeros
+        new = new if stream is None else _on_stream(new, stream)
+        digests = new((max(n_digests, 1), 4), dtype=torch.uint64, device=leaves.device)
     if cap is None:
-        cap = _new((n_caps, 4), leaves.device, stream, zero=not written)
+        new = torch.empty if written else torch.zeros
+        new = new if stream is None else _on_stream(new, stream)
+        cap = new((n_caps, 4), dtype=torch.uint64, device=leaves.device)
     capi.check(capi.LIB.zk_merkle_async(digests.data_ptr(), cap.data_ptr(), leaves.data_ptr(), n_digests, n_caps,
                                         n_leaves, w, cap_height, hash_type, _stream_ptr(stream)))
     return digests, cap
@@ -364,14 +380,15 @@ def merkle_open(leaves, digests, cap_height: int, indices, stream=None):
     n_leaves, w = leaves.shape
     # A copy from the host is complete when it returns, whatever stream it took; work on `stream` does
     # not hold it up.  A conversion on the device is only ordered where it runs.
-    with _on(stream if indices.is_cuda else None):
+    with _HERE if stream is None or not indices.is_cuda else _on(stream):
         idx = indices.to(device=leaves.device, dtype=torch.int64).contiguous().view(torch.uint64)
     if stream is not None:
         idx.record_stream(_torch_stream(stream))
     q = idx.numel()
     depth = (n_leaves >> cap_height).bit_length() - 1
-    rows = _new((q, w), leaves.device, stream)
-    sib = _new((q, depth, 4), leaves.device, stream)
+    new = torch.empty if stream is None else _on_stream(torch.empty, stream)
+    rows = new((q, w), dtype=torch.uint64, device=leaves.device)
+    sib = new((q, depth, 4), dtype=torch.uint64, device=leaves.device)
     capi.check(capi.LIB.zk_merkle_open_async(leaves.data_ptr(), digests.data_ptr(), n_leaves, w, cap_height,
                                              idx.data_ptr(), q, rows.data_ptr(), sib.data_ptr(), _stream_ptr(stream)))
     return rows, sib
@@ -390,7 +407,8 @@ def fri_fold(coeffs, arity_bits: int, beta, *, interleaved: bool = False, out=No
     n = coeffs.shape[0] if interleaved else coeffs.shape[1]
     assert coeffs.shape == ((n, 2) if interleaved else (2, n))
     if out is None:
-        out = _new((2, n >> arity_bits), coeffs.device, stream)
+        new = torch.empty if stream is None else _on_stream(torch.empty, stream)
+        out = new((2, n >> arity_bits), dtype=torch.uint64, device=coeffs.device)
     capi.check(capi.LIB.zk_fri_fold_async(out.data_ptr(), coeffs.data_ptr(), n, arity_bits, int(beta[0]) % P,
                                           int(beta[1]) % P, int(interleaved), _stream_ptr(stream)))
     return out
@@ -432,7 +450,7 @@ def fri_commit(coeffs, rate_bits: int, arity_bits, cap_height: int, challenge, h
         view = leaves.view((n << rate_bits) >> ab, 2 << ab)
         dig, cap = merkle_tree(view, cap_height, hash_type, stream=stream)
         rnd = FriRound(view, dig, cap, ab, shift)
-        with _on(stream):
+        with _HERE if stream is None else _on(stream):
             cap_host = cap.cpu().numpy()  # waits for the round
         rnd.beta = challenge(i, cap_host)
         rounds.append(rnd)
