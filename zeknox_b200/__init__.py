@@ -152,14 +152,13 @@ def lde_leaves_coset(coeffs, rate_bits: int, coset_gen: int, out=None, stream=No
 class CommitBuffers:
     """Device outputs of one commit: leaves (N, B), digests (2(N - 2^cap), 4), cap (2^cap, 4)."""
 
-    def __init__(self, n_leaves: int, width: int, cap_height: int, device="cuda", stream=None):
+    def __init__(self, n_leaves: int, width: int, cap_height: int, device="cuda"):
         import torch
 
-        new = torch.empty if stream is None else _on_stream(torch.empty, stream)
         nd, nc = merkle_sizes(n_leaves, cap_height)
-        self.leaves = new((n_leaves, width), dtype=torch.uint64, device=device)
-        self.digests = new((max(nd, 1), 4), dtype=torch.uint64, device=device)
-        self.cap = new((nc, 4), dtype=torch.uint64, device=device)
+        self.leaves = torch.empty((n_leaves, width), dtype=torch.uint64, device=device)
+        self.digests = torch.empty((max(nd, 1), 4), dtype=torch.uint64, device=device)
+        self.cap = torch.empty((nc, 4), dtype=torch.uint64, device=device)
 
 
 def commit(coeffs, rate_bits: int, cap_height: int, hash_type: int = HashPoseidon, out: CommitBuffers | None = None,
@@ -168,7 +167,13 @@ def commit(coeffs, rate_bits: int, cap_height: int, hash_type: int = HashPoseido
     b, n = coeffs.shape
     lg_n = n.bit_length() - 1
     if out is None:
-        out = CommitBuffers(n << rate_bits, b, cap_height, coeffs.device, stream)
+        with _HERE if stream is None else _on(stream):
+            out = CommitBuffers(n << rate_bits, b, cap_height, coeffs.device)
+        if stream is not None:
+            import torch
+
+            for t in (out.leaves, out.digests, out.cap):
+                t.record_stream(torch.cuda.current_stream(coeffs.device))
     capi.check(capi.LIB.zk_commit_async(coeffs.data_ptr(), lg_n, rate_bits, b, cap_height, hash_type,
                                         out.leaves.data_ptr(), out.digests.data_ptr(), out.cap.data_ptr(),
                                         _stream_ptr(stream)))
