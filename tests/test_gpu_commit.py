@@ -260,6 +260,36 @@ def test_commit_batch_graph_replays_bit_exact(zk, oracle):
             assert torch.equal(alone.leaves.view(torch.int64), o.leaves.view(torch.int64))
 
 
+def test_helpers_on_a_given_stream_alone_and_captured(zk, oracle):
+    """commit, lde and merkle_tree that allocate on a given stream: with work pending on the current one, and
+    inside a graph captured on that stream."""
+    import torch
+
+    b, lg_n, rate, cap_h = 9, 11, 2, 2
+    x = oracle.field_elems(4300, b << lg_n)
+    rows = oracle.batch_lde(x, lg_n, rate, b)
+    leaves = oracle.transpose_rev(rows, lg_n + rate, b)
+    dig, cap = oracle.merkle_fill(leaves, b, cap_h, oracle.HASH_POSEIDON)
+    d, side = _dev(x).view(b, -1), torch.cuda.Stream()
+    y = torch.ones(4096, 4096, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(50):
+        y = y @ y * 2.0**-12
+    out = zk.commit(d, rate, cap_h, stream=side)
+    got = zk.lde(d, rate, stream=side)
+    torch.cuda.synchronize()
+    assert np.array_equal(out.leaves.cpu().numpy().reshape(-1), leaves)
+    assert np.array_equal(out.digests.cpu().numpy().reshape(-1), dig)
+    assert np.array_equal(out.cap.cpu().numpy().reshape(-1), cap) and np.array_equal(got.cpu().numpy().reshape(-1), rows)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side), torch.cuda.graph(graph, stream=side):
+        lv = zk.lde_leaves(d, rate, stream=side)
+        gd, gc = zk.merkle_tree(lv, cap_h, stream=side)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.array_equal(gd.cpu().numpy().reshape(-1), dig) and np.array_equal(gc.cpu().numpy().reshape(-1), cap)
+
+
 def test_autotuner_choices_keep_outputs_bit_exact(zk, oracle):
     """Tuning the LDE -> leaves stage changes only how it runs: commits of the
     tuned shapes equal the untuned ones, and a tuned shape is not re-timed."""
